@@ -358,6 +358,10 @@ void push_pa(espp_system* s) {
   s->paHostValid = true;
 }
 
+// A copy from pageable memory or a memset on the legacy stream may still be running when the
+// call returns, and the systems' streams do not wait for that stream.
+void settle_uploads() { cuda_check(cudaStreamSynchronize(cudaStreamLegacy), "upload"); }
+
 // Host copy of every particle in storage order.
 struct HostParticles {
   std::vector<int64_t> id;
@@ -369,8 +373,9 @@ template <class T>
 void copy_soa_down(espp_system* s, std::vector<T>& out, const T* dsrc, int comps) {
   std::vector<T> tmp((size_t)comps * s->cap);
   if (s->cap)
-    cuda_check(cudaMemcpy(tmp.data(), dsrc, sizeof(T) * tmp.size(), cudaMemcpyDeviceToHost),
-               "download");
+    cuda_check(cudaMemcpyAsync(tmp.data(), dsrc, sizeof(T) * tmp.size(), cudaMemcpyDeviceToHost,
+                               s->st), "download");
+  sync(s);
   out.resize((size_t)comps * s->n);
   for (int i = 0; i < s->n; ++i)
     for (int c = 0; c < comps; ++c) out[(size_t)comps * i + c] = tmp[(size_t)c * s->cap + i];
@@ -394,8 +399,8 @@ void copy_soa_up(espp_system* s, T* ddst, const std::vector<T>& in, int comps) {
   std::vector<T> tmp((size_t)comps * s->cap, T(0));
   for (int i = 0; i < s->n; ++i)
     for (int c = 0; c < comps; ++c) tmp[(size_t)c * s->cap + i] = in[(size_t)comps * i + c];
-  cuda_check(cudaMemcpy(ddst, tmp.data(), sizeof(T) * tmp.size(), cudaMemcpyHostToDevice),
-             "upload");
+  cuda_check(cudaMemcpyAsync(ddst, tmp.data(), sizeof(T) * tmp.size(), cudaMemcpyHostToDevice,
+                             s->st), "upload");
 }
 
 void free_buffers(espp_system* s) {
@@ -433,14 +438,14 @@ void upload(espp_system* s, const HostParticles& h) {
     s->pcell = dalloc<int32_t>(cap);
     s->nn = dalloc<int32_t>(cap);
     s->nnZero = dalloc<int32_t>(cap);
-    cuda_check(cudaMemset(s->nnZero, 0, sizeof(int32_t) * cap), "memset");
+    cuda_check(cudaMemsetAsync(s->nnZero, 0, sizeof(int32_t) * cap, s->st), "memset");
     s->ffix = dalloc<long long>(3 * (size_t)cap);
     s->f64 = dalloc<double>(3 * (size_t)cap);
     s->ftot = dalloc<double>(3 * (size_t)cap);
     s->scr.cellOf = dalloc<int32_t>(cap);
     s->scr.slot = dalloc<int32_t>(cap);
     s->scr.perm = dalloc<int32_t>(cap);
-    cuda_check(cudaMemset(s->nn, 0, sizeof(int32_t) * cap), "memset");
+    cuda_check(cudaMemsetAsync(s->nn, 0, sizeof(int32_t) * cap, s->st), "memset");
     s->K = 0;
     dfree(s->nl);
     s->bKb = 0;
@@ -460,8 +465,8 @@ void upload(espp_system* s, const HostParticles& h) {
   std::vector<double> f = h.f;
   if (f.size() != h.x.size()) f.assign(h.x.size(), 0.0);
   copy_soa_up(s, s->ftot, f, 3);
-  cuda_check(cudaMemset(s->ffix, 0, sizeof(long long) * 3 * s->cap), "memset");
-  cuda_check(cudaMemset(s->f64, 0, sizeof(double) * 3 * s->cap), "memset");
+  cuda_check(cudaMemsetAsync(s->ffix, 0, sizeof(long long) * 3 * s->cap, s->st), "memset");
+  cuda_check(cudaMemsetAsync(s->f64, 0, sizeof(double) * 3 * s->cap, s->st), "memset");
   s->binned = false;
   ensure_mlp_scratch(s);
 }
@@ -490,7 +495,7 @@ void rebuild_id_tables(espp_system* s) {
                            std::to_string(span) + ")");
   s->idSpan = (int)span;
   s->id2idx = dalloc<int32_t>(span);
-  cuda_check(cudaMemset(s->id2idx, 0xff, sizeof(int32_t) * span), "memset");
+  cuda_check(cudaMemsetAsync(s->id2idx, 0xff, sizeof(int32_t) * span, s->st), "memset");
   auto csr = [&](const std::vector<std::pair<int64_t, int64_t>>& pairs, int32_t*& dstart,
                  int64_t*& dids) {
     std::vector<int32_t> start(span + 1, 0);
@@ -507,10 +512,10 @@ void rebuild_id_tables(espp_system* s) {
     }
     dstart = dalloc<int32_t>(span + 1);
     dids = dalloc<int64_t>(ids.size());
-    cuda_check(cudaMemcpy(dstart, start.data(), sizeof(int32_t) * (span + 1),
-                          cudaMemcpyHostToDevice), "upload");
-    cuda_check(cudaMemcpy(dids, ids.data(), sizeof(int64_t) * ids.size(),
-                          cudaMemcpyHostToDevice), "upload");
+    cuda_check(cudaMemcpyAsync(dstart, start.data(), sizeof(int32_t) * (span + 1),
+                          cudaMemcpyHostToDevice, s->st), "upload");
+    cuda_check(cudaMemcpyAsync(dids, ids.data(), sizeof(int64_t) * ids.size(),
+                          cudaMemcpyHostToDevice, s->st), "upload");
   };
   for (auto& b : s->bonds)
     if (b.first < s->idMin || b.second < s->idMin || b.first - s->idMin >= span ||
@@ -550,23 +555,25 @@ void rebuild_id_tables(espp_system* s) {
     s->tripStart = dalloc<int32_t>(span + 1);
     s->tripEntry = dalloc<int32_t>(entry.size());
     s->tripF = dalloc<double>(6 * nt);
-    cuda_check(cudaMemcpy(s->d_triples, ids.data(), sizeof(int64_t) * ids.size(),
-                          cudaMemcpyHostToDevice), "upload");
-    cuda_check(cudaMemcpy(s->tripStart, start.data(), sizeof(int32_t) * (span + 1),
-                          cudaMemcpyHostToDevice), "upload");
-    cuda_check(cudaMemcpy(s->tripEntry, entry.data(), sizeof(int32_t) * entry.size(),
-                          cudaMemcpyHostToDevice), "upload");
+    cuda_check(cudaMemcpyAsync(s->d_triples, ids.data(), sizeof(int64_t) * ids.size(),
+                          cudaMemcpyHostToDevice, s->st), "upload");
+    cuda_check(cudaMemcpyAsync(s->tripStart, start.data(), sizeof(int32_t) * (span + 1),
+                          cudaMemcpyHostToDevice, s->st), "upload");
+    cuda_check(cudaMemcpyAsync(s->tripEntry, entry.data(), sizeof(int32_t) * entry.size(),
+                          cudaMemcpyHostToDevice, s->st), "upload");
   }
   std::vector<uint8_t> le(span, 0);
   for (int64_t id : s->langExclIds)
     if (id >= s->idMin && id - s->idMin < span) le[id - s->idMin] = 1;
   s->langExcl = dalloc<uint8_t>(span);
-  cuda_check(cudaMemcpy(s->langExcl, le.data(), span, cudaMemcpyHostToDevice), "upload");
+  cuda_check(cudaMemcpyAsync(s->langExcl, le.data(), span, cudaMemcpyHostToDevice, s->st),
+             "upload");
   if (!s->haloIds.empty()) {
     std::vector<uint8_t> hl(span, 0);
     for (int64_t id : s->haloIds) hl[id - s->idMin] = 1;
     s->halo = dalloc<uint8_t>(span);
-    cuda_check(cudaMemcpy(s->halo, hl.data(), span, cudaMemcpyHostToDevice), "upload");
+    cuda_check(cudaMemcpyAsync(s->halo, hl.data(), span, cudaMemcpyHostToDevice, s->st),
+               "upload");
   }
   s->idDirty = false;
   s->binned = false;
@@ -809,10 +816,10 @@ void upload_lj(espp_system* s) {
   dfree(s->d_ljf);
   s->d_lj = dalloc<LJPair>(std::max<size_t>(compact.size(), 1));
   s->d_ljf = dalloc<LJPairF>(std::max<size_t>(compact.size(), 1));
-  cuda_check(cudaMemcpy(s->d_lj, t.p, sizeof(LJPair) * compact.size(), cudaMemcpyHostToDevice),
-             "upload");
-  cuda_check(cudaMemcpy(s->d_ljf, f.data(), sizeof(LJPairF) * compact.size(),
-                        cudaMemcpyHostToDevice), "upload");
+  cuda_check(cudaMemcpyAsync(s->d_lj, t.p, sizeof(LJPair) * compact.size(),
+                             cudaMemcpyHostToDevice, s->st), "upload");
+  cuda_check(cudaMemcpyAsync(s->d_ljf, f.data(), sizeof(LJPairF) * compact.size(),
+                        cudaMemcpyHostToDevice, s->st), "upload");
   s->lj.single = (nt == 1 && compact[0].set) ? 1 : 0;
 }
 
@@ -856,15 +863,15 @@ void upload_tabs(espp_system* s) {
   if (!descs.empty()) {
     s->d_tabs = dalloc<TabDesc>(descs.size());
     s->d_tabCoef = dalloc<double>(coef.size());
-    cuda_check(cudaMemcpy(s->d_tabs, descs.data(), sizeof(TabDesc) * descs.size(),
-                          cudaMemcpyHostToDevice), "upload");
-    cuda_check(cudaMemcpy(s->d_tabCoef, coef.data(), sizeof(double) * coef.size(),
-                          cudaMemcpyHostToDevice), "upload");
+    cuda_check(cudaMemcpyAsync(s->d_tabs, descs.data(), sizeof(TabDesc) * descs.size(),
+                          cudaMemcpyHostToDevice, s->st), "upload");
+    cuda_check(cudaMemcpyAsync(s->d_tabCoef, coef.data(), sizeof(double) * coef.size(),
+                          cudaMemcpyHostToDevice, s->st), "upload");
   }
   if (nt > 0) {
     s->d_tabPair = dalloc<int32_t>(pairMap.size());
-    cuda_check(cudaMemcpy(s->d_tabPair, pairMap.data(), sizeof(int32_t) * pairMap.size(),
-                          cudaMemcpyHostToDevice), "upload");
+    cuda_check(cudaMemcpyAsync(s->d_tabPair, pairMap.data(), sizeof(int32_t) * pairMap.size(),
+                          cudaMemcpyHostToDevice, s->st), "upload");
   }
   s->tabNT = nt;
   s->tabBond = bondIdx;
@@ -1756,14 +1763,14 @@ int espp_system_create(const double box[3], double skin, const int32_t cell_grid
     s->cellStart = dalloc<int32_t>(ncells + 1);
     s->scr.cellCount = dalloc<int32_t>(ncells);
     s->scr.tileSum = dalloc<int32_t>(scan_tiles((int)ncells) + 1);
-    cuda_check(cudaMemset(s->cellStart, 0, sizeof(int32_t) * (ncells + 1)), "memset");
+    cuda_check(cudaMemsetAsync(s->cellStart, 0, sizeof(int32_t) * (ncells + 1), s->st), "memset");
     s->err = dalloc<unsigned>(1);
     s->ctr = dalloc<DevCounters>(1);
     s->d_pa = dalloc<ParticleArrays>(2);
     s->obs = dalloc<double>(8);
-    cuda_check(cudaMemset(s->err, 0, sizeof(unsigned)), "memset");
-    cuda_check(cudaMemset(s->ctr, 0, sizeof(DevCounters)), "memset");
-    cuda_check(cudaMemset(s->d_pa, 0, 2 * sizeof(ParticleArrays)), "memset");
+    cuda_check(cudaMemsetAsync(s->err, 0, sizeof(unsigned), s->st), "memset");
+    cuda_check(cudaMemsetAsync(s->ctr, 0, sizeof(DevCounters), s->st), "memset");
+    cuda_check(cudaMemsetAsync(s->d_pa, 0, 2 * sizeof(ParticleArrays), s->st), "memset");
     cuda_check(cudaMallocHost(&s->hctr, sizeof(DevCounters)), "pinned counters");
     if (const char* g = std::getenv("ESPP_B200_GRAPH")) s->useGraph = std::atoi(g) != 0;
     if (const char* b = std::getenv("ESPP_B200_BRICK")) s->brickAllowed = std::atoi(b) != 0;
@@ -2080,7 +2087,8 @@ int espp_vl_pairs(espp_system* s, int64_t capn, int64_t* pairs, int64_t* npairs)
     int64_t* doff = dalloc<int64_t>(s->n);
     int64_t* dout = dalloc<int64_t>(2 * std::max<int64_t>(t, 1));
     std::vector<int64_t> out(2 * std::max<int64_t>(t, 1));
-    cudaMemcpy(doff, off.data(), sizeof(int64_t) * s->n, cudaMemcpyHostToDevice);
+    cuda_check(cudaMemcpyAsync(doff, off.data(), sizeof(int64_t) * s->n, cudaMemcpyHostToDevice,
+                               s->st), "upload");
     if (s->brickOn)
       launch_pair_write_brick(d, doff, counts, dout, s->st);
     else
@@ -2719,6 +2727,7 @@ int espp_mlp_create(double rc, double r0, espp_mlp** out) {
                "upload");
     cuda_check(cudaMemcpy(m->scale, one.data(), sizeof(float) * kMlpK, cudaMemcpyHostToDevice),
                "upload");
+    settle_uploads();
     *out = m.release();
   });
 }
@@ -2755,6 +2764,7 @@ int espp_mlp_set_params(espp_mlp* m, int64_t n, const double* theta) {
     std::vector<float> h(theta, theta + n);
     cuda_check(cudaMemcpy(m->theta, h.data(), sizeof(float) * n, cudaMemcpyHostToDevice),
                "upload");
+    settle_uploads();
   });
 }
 
@@ -2779,6 +2789,7 @@ int espp_mlp_set_norm(espp_mlp* m, const double* shift, const double* scale) {
                "upload");
     cuda_check(cudaMemcpy(m->scale, b.data(), sizeof(float) * kMlpK, cudaMemcpyHostToDevice),
                "upload");
+    settle_uploads();
   });
 }
 
