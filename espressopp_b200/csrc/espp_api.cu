@@ -152,7 +152,7 @@ struct espp_system {
   // brick path of the Verlet list and pair kernels (BrickView)
   bool brickAllowed = false;  // ESPP_B200_BRICK=1 selects the brick form
   bool brickBuild = false;    // the global-form list is built by brick windows
-                              // (ESPP_B200_BRICK_BUILD=1) instead of the per-cell lanes
+                              // (ESPP_B200_BRICK_BUILD=1) instead of launch_build_nl's
   bool brickBuildUsed = false;  // the current global-form list came from the brick build
   bool brickOn = false;       // the current list is in the brick form
   int brickB[3] = {0, 0, 0};  // brick extent in cells (0: chosen from the density)
@@ -612,11 +612,9 @@ void bin(espp_system* s, bool fold) {
     return;
   }
   launch_fold_bin(d, s->scr, fold, s->st);
-  launch_sort_cells(d, s->scr, s->st);
-  launch_gather(d, s->scr, s->st);  // gathers into pa[1] and swaps on the device
+  launch_sort_cells(d, s->scr, s->st);  // moves into pa[1] and swaps on the device
   s->paHostValid = false;
   s->xrelFresh = true;
-  launch_id_map(d, s->st);
   cuda_check(cudaGetLastError(), "re-binning kernels");
   s->binned = true;
   s->listValid = false;
@@ -723,8 +721,8 @@ bool grow_brick_window(espp_system* s) {
   return true;
 }
 
-// The per-particle global form: built by brick windows when the grid allows (every
-// candidate read once per brick from shared memory), else by the per-cell lane kernel.
+// The per-particle global form: built by brick windows where those were asked for
+// (every candidate read once per brick from shared memory), else by launch_build_nl.
 void build_list_plain(espp_system* s, double cutsq) {
   if (s->K == 0 || !s->nl) {
     s->K = estimate_K(s);
@@ -987,10 +985,10 @@ void collect_phases(espp_system* s) {
   s->evUsed = 0;
 }
 
-// rebuild = fold/bin (fold_bin, scan, scatter, sort, gather, id map) + Verlet list
+// rebuild = fold/bin (fold_bin, scan, scatter, sort and move) + Verlet list
 void timed_decompose(espp_system* s) {
   {
-    PhaseScope ps(s, kPhRebuild, 10);
+    PhaseScope ps(s, kPhRebuild, resort_launches(s->view()));
     bin(s, true);
   }
   check_err(s);
@@ -1047,8 +1045,6 @@ void launch_rebuild_kernels(espp_system* s, cudaStream_t st) {
   DevView d = s->view();
   launch_fold_bin(d, s->scr, true, st);
   launch_sort_cells(d, s->scr, st);
-  launch_gather(d, s->scr, st);
-  launch_id_map(d, st);
   if (s->has_vl) {
     const double cv = s->vl_cut + s->skin;
     if (s->brickOn || s->brickBuildUsed) {
@@ -1062,7 +1058,7 @@ void launch_rebuild_kernels(espp_system* s, cudaStream_t st) {
 void launch_force_kernel(espp_system* s, cudaStream_t st) { launch_all_forces(s, st); }
 
 // Adds to graph g one WHILE node (no dependencies) running the step loop of s:
-// WHILE(remaining) { decide; IF(re-sort) { fold, bin, sort, gather, swap, id map, list };
+// WHILE(remaining) { decide; IF(re-sort) { fold + bin, scan, scatter, sort + move, list };
 //                    force; integrate2 + integrate1 }
 void add_step_loop(espp_system* s, cudaGraph_t g, const IntegrateArgs& ai) {
   cudaGraphConditionalHandle hWhile, hIf;
@@ -1304,12 +1300,12 @@ void graph_loop_done(espp_system* s, int64_t nsteps) {
   s->step += nsteps;
   s->nResorts = c.resorts;
   s->builds += c.resorts;
-  // kernels launched by the graph: decide + force + integrate per step, and zero,
-  // fold/bin, scan (3), scatter, in-cell sort, gather, swap, id map (+ list) per re-sort
+  // kernels launched by the graph: decide + force + integrate per step, and fold/bin, scan
+  // (1 or 2), scatter, sort, move (+ list) per re-sort
   s->phaseLaunches[kPhOther] += nsteps;
   s->phaseLaunches[kPhForce] += nsteps;
   s->phaseLaunches[kPhIntegrate] += nsteps;
-  s->phaseLaunches[kPhRebuild] += c.resorts * 10;
+  s->phaseLaunches[kPhRebuild] += c.resorts * resort_launches(s->view());
   s->phaseLaunches[kPhList] += s->has_vl ? c.resorts : 0;
   s->paHostValid = false;
 }
@@ -1603,6 +1599,7 @@ void destroy(espp_system* s) {
   dfree(s->cellStart);
   dfree(s->scr.cellCount);
   dfree(s->scr.tileSum);
+  dfree(s->scr.ticket);
   dfree(s->id2idx);
   dfree(s->bondStart);
   dfree(s->bondPartner);
@@ -1763,6 +1760,9 @@ int espp_system_create(const double box[3], double skin, const int32_t cell_grid
     s->cellStart = dalloc<int32_t>(ncells + 1);
     s->scr.cellCount = dalloc<int32_t>(ncells);
     s->scr.tileSum = dalloc<int32_t>(scan_tiles((int)ncells) + 1);
+    s->scr.ticket = dalloc<unsigned>(1);
+    cuda_check(cudaMemsetAsync(s->scr.cellCount, 0, sizeof(int32_t) * ncells, s->st), "memset");
+    cuda_check(cudaMemsetAsync(s->scr.ticket, 0, sizeof(unsigned), s->st), "memset");
     cuda_check(cudaMemsetAsync(s->cellStart, 0, sizeof(int32_t) * (ncells + 1), s->st), "memset");
     s->err = dalloc<unsigned>(1);
     s->ctr = dalloc<DevCounters>(1);

@@ -197,16 +197,16 @@ struct DevView {
 struct RebuildScratch {
   int32_t* cellOf;    // cap: cell of particle (unsorted order)
   int32_t* slot;      // cap: arrival slot inside its cell
-  int32_t* cellCount; // ncells
+  int32_t* cellCount; // ncells, zero between binnings
   int32_t* perm;      // cap: sorted position -> old row
-  int32_t* tileSum;   // scan_tiles(ncells): per-tile sums / offsets of the cell scan
+  int32_t* tileSum;   // scan_tiles(ncells): per-tile sums of the cell scan
+  unsigned* ticket;   // blocks of the moving kernel that have finished, 0 between launches
 };
 
 // launchers (espp_kernels.cu)
 void launch_fold_bin(const DevView& d, RebuildScratch& s, bool fold, cudaStream_t st);
 void launch_sort_cells(const DevView& d, RebuildScratch& s, cudaStream_t st);
-void launch_gather(const DevView& d, const RebuildScratch& s, cudaStream_t st);
-void launch_id_map(const DevView& d, cudaStream_t st);
+int resort_launches(const DevView& d);  // kernels of one re-sort without the list build
 // Verlet list in the global form; fresh: the particles were binned at their current
 // positions (the run form may then be used).
 void launch_build_nl(const DevView& d, double cutsq, bool fresh, cudaStream_t st);

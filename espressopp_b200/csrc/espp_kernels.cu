@@ -1,21 +1,25 @@
 // espp_kernels.cu - sm_100a kernels of the short-range MD step.
 //
-//  re-binning     k_fold_bin -> k_scan_cells -> k_scatter -> k_sort_in_cell -> k_gather
+//  re-binning     k_fold_bin -> k_scan_* -> k_scatter -> k_sort_cells (-> k_move)
 //                 (storage::DomainDecomposition::decomposeRealParticles, one node)
-//  Verlet list    k_build_nl_run (runs of 32 particles of a row of cells, candidates
-//                 filtered against the group's bounding box) / k_build_nl_lane (one warp
-//                 per cell): FP32 test with the reference's FP64 ghost-shift arithmetic
-//                 near the cutoff, full per-particle list (VerletList::_rebuildUsingBuffers)
+//  Verlet list    k_build_block (a block per run of 32 particles of a row of cells,
+//                 candidates filtered against the run's bounding box) / k_build_nl_run (one
+//                 warp per run, lists of any length): FP32 test with the reference's FP64
+//                 ghost-shift arithmetic near the cutoff, full per-particle list
+//                 (VerletList::_rebuildUsingBuffers)
 //  forces         k_force_mixed (FP32 on box-wrapped int32 coordinates, int64 2^-32
 //                 fixed-point output) / k_force_fp64 (plain FP64); LJ + FENE fused
 //  integrator     k_integrate: aftCalcF (Langevin, CapForce) + integrate2 of step n +
-//                 integrate1 of step n+1 in one pass over the particle arrays
+//                 integrate1 of step n+1 in one pass over the particle arrays; k_steps: every
+//                 step of a small system up to the next re-sort in one launch
 //  observables    FP64 energy / virial / kinetic with fixed-order block reductions
 #include <math.h>
 #include <stddef.h>
 #include <stdint.h>
 #include <stdlib.h>
 #include <string.h>
+
+#include <type_traits>
 
 #include "espp_device.h"
 #include "espp_internal.h"
@@ -68,7 +72,9 @@ __device__ __forceinline__ void langevin_uniforms(uint64_t seed, int64_t id, int
 
 // ---- re-binning --------------------------------------------------------------------
 
-// OrthorhombicBC::foldCoordinate + CellGrid::mapPositionToCellChecked/Clipped.
+// OrthorhombicBC::foldCoordinate + CellGrid::mapPositionToCellChecked/Clipped.  Bound by
+// memory: positions and images go back only where a fold changed them (20.6 us, 16.3 without
+// the other writes, at a million particles).
 __global__ void k_fold_bin(DevView d, RebuildScratch s, int fold) {
   const ParticleArrays a = d.pa[0];
   int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -85,9 +91,11 @@ __global__ void k_fold_bin(DevView d, RebuildScratch s, int fold) {
         q = 0.0;
       }
       int tmp = (int)q;
-      a.img[(size_t)k * d.cap + i] += tmp;
-      x = __dsub_rn(x, __dmul_rn((double)tmp, d.L[k]));
-      a.x[(size_t)k * d.cap + i] = x;
+      if (tmp != 0) {  // most particles are inside the box: nothing to write
+        a.img[(size_t)k * d.cap + i] += tmp;
+        x = __dsub_rn(x, __dmul_rn((double)tmp, d.L[k]));
+        a.x[(size_t)k * d.cap + i] = x;
+      }
     }
     double lpos = x;
     double t = __dmul_rn(lpos, d.invCellSize[k]);
@@ -112,8 +120,9 @@ __global__ void k_fold_bin(DevView d, RebuildScratch s, int fold) {
   s.slot[i] = atomicAdd(&s.cellCount[cell], 1);
 }
 
-// Exclusive scan of the cell counts into cellStart, in three passes: block sums, a
-// scan of the block sums (one block), then each block's scan plus its offset.
+// Exclusive scan of the cell counts into cellStart: sums of tiles of cells, then each
+// tile's scan behind the sum of the tiles before it (one tile: the second pass alone).  The
+// counts are left zero for the next binning.
 constexpr int kScanBlock = 1024;
 constexpr int kScanItems = 4;
 constexpr int kScanTile = kScanBlock * kScanItems;
@@ -156,35 +165,27 @@ __global__ void __launch_bounds__(kScanBlock) k_scan_tiles(const int32_t* __rest
   if (threadIdx.x == 0) tile_sum[blockIdx.x] = total;
 }
 
-__global__ void __launch_bounds__(kScanBlock) k_scan_tile_sums(int32_t* __restrict__ tile_sum,
-                                                                int ntiles) {
-  __shared__ int sm[32];
-  int carry = 0;
-  for (int b = 0; b < ntiles; b += kScanBlock) {
-    const int t = b + (int)threadIdx.x;
-    const int v = t < ntiles ? tile_sum[t] : 0;
-    int total;
-    const int e = block_exclusive_scan(v, sm, total);
-    if (t < ntiles) tile_sum[t] = carry + e;
-    carry += total;
-  }
-}
-
-__global__ void __launch_bounds__(kScanBlock) k_scan_apply(const int32_t* __restrict__ count,
-                                                            int n,
-                                                            const int32_t* __restrict__ tile_off,
+__global__ void __launch_bounds__(kScanBlock) k_scan_apply(int32_t* __restrict__ count, int n,
+                                                            const int32_t* __restrict__ tile_sum,
                                                             int32_t* __restrict__ start) {
   __shared__ int sm[32];
+  __shared__ int s_before;
+  int before = 0;
+  for (int t = threadIdx.x; t < (int)blockIdx.x; t += blockDim.x) before += tile_sum[t];
+  int total;
+  block_exclusive_scan(before, sm, total);
+  if (threadIdx.x == 0) s_before = total;
+  __syncthreads();
   const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
   int c[kScanItems];
   int v = 0;
 #pragma unroll
   for (int k = 0; k < kScanItems; ++k) {
     c[k] = (base + k < n) ? count[base + k] : 0;
+    if (base + k < n) count[base + k] = 0;
     v += c[k];
   }
-  int total;
-  int run = block_exclusive_scan(v, sm, total) + tile_off[blockIdx.x];
+  int run = block_exclusive_scan(v, sm, total) + s_before;
 #pragma unroll
   for (int k = 0; k < kScanItems; ++k) {
     if (base + k < n) start[base + k] = run;
@@ -202,16 +203,12 @@ __global__ void k_scatter(DevView d, RebuildScratch s) {
 // Order inside a cell: by the Morton code of the particle's 8 x 8 x 8 sub-cell, then by
 // id.  The layout is independent of the atomic arrival order above, and consecutive
 // particles (the lanes of a force warp) sit close together, so their neighbour lists
-// overlap and their coordinate gathers share cache lines.  One warp per cell: each lane
-// takes one particle and its rank among the cell's keys is its new slot (cells with
-// more than 32 particles are sorted by insertion on lane 0).
+// overlap and their coordinate gathers share cache lines.
 __device__ __forceinline__ unsigned spread3(unsigned v) {  // bits b2 b1 b0 -> b2..b1..b0
   return (v & 1u) | ((v & 2u) << 2) | ((v & 4u) << 4);
 }
 __device__ __forceinline__ uint64_t in_cell_key(const DevView& d, const ParticleArrays& a, int v,
-                                                int c) {
-  const int cx = c % d.nc[0], cy = (c / d.nc[0]) % d.nc[1], cz = c / (d.nc[0] * d.nc[1]);
-  const int cc[3] = {cx, cy, cz};
+                                                const int (&cc)[3]) {
   unsigned q[3];
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
@@ -225,75 +222,114 @@ __device__ __forceinline__ uint64_t in_cell_key(const DevView& d, const Particle
   return (morton << 54) | (uint64_t)(a.id[v] - d.idMin);
 }
 
-__global__ void k_sort_in_cell(DevView d, RebuildScratch s) {
-  const ParticleArrays a = d.pa[0];
-  const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (c >= d.ncells) return;
-  const int b = d.cellStart[c], e = d.cellStart[c + 1];
-  const int n = e - b;
-  if (n <= 1) return;
-  if (n <= 32) {
-    const int v = lane < n ? s.perm[b + lane] : 0;
-    const uint64_t key = lane < n ? in_cell_key(d, a, v, c) : UINT64_MAX;
-    int rank = 0;
-    for (int m = 0; m < n; ++m) {
-      const uint64_t km = __shfl_sync(0xffffffffu, key, m);
-      rank += km < key;
-    }
-    __syncwarp();
-    if (lane < n) s.perm[b + rank] = v;
-    return;
-  }
-  if (lane == 0) {
-    for (int k = b + 1; k < e; ++k) {
-      const int v = s.perm[k];
-      const uint64_t key = in_cell_key(d, a, v, c);
-      int m = k - 1;
-      while (m >= b && in_cell_key(d, a, s.perm[m], c) > key) {
-        s.perm[m + 1] = s.perm[m];
-        --m;
-      }
-      s.perm[m + 1] = v;
-    }
-  }
-}
-
-__global__ void k_gather(DevView d, RebuildScratch s) {
-  const ParticleArrays src = d.pa[0], dst = d.pa[1];
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= d.n) return;
-  int o = s.perm[k];
+// Row k of the other copy of the arrays from row o, with everything derived from a row:
+// packed and cell-relative coordinates, cell, id map.
+__device__ __forceinline__ void move_row(const DevView& d, const RebuildScratch& s,
+                                         const ParticleArrays& src, const ParticleArrays& dst,
+                                         int o, int k) {
   double p[3];
 #pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    p[c] = src.x[(size_t)c * d.cap + o];
-    dst.x[(size_t)c * d.cap + k] = p[c];
-    dst.v[(size_t)c * d.cap + k] = src.v[(size_t)c * d.cap + o];
-    dst.img[(size_t)c * d.cap + k] = src.img[(size_t)c * d.cap + o];
+  for (int e = 0; e < 3; ++e) {
+    p[e] = src.x[(size_t)e * d.cap + o];
+    dst.x[(size_t)e * d.cap + k] = p[e];
+    dst.v[(size_t)e * d.cap + k] = src.v[(size_t)e * d.cap + o];
+    dst.img[(size_t)e * d.cap + k] = src.img[(size_t)e * d.cap + o];
   }
-  int ty = src.type[o];
-  dst.id[k] = src.id[o];
+  const int ty = src.type[o];
+  const int64_t id = src.id[o];
+  dst.id[k] = id;
   dst.type[k] = ty;
   dst.mass[k] = src.mass[o];
   const int cell = s.cellOf[o];
   d.pcell[k] = cell;
   d.posq[k] = fixed_coords(d, p[0], p[1], p[2], ty);
-  const int cx = cell % d.nc[0], cy = (cell / d.nc[0]) % d.nc[1], cz = cell / (d.nc[0] * d.nc[1]);
+  const int cx = cell % d.nc[0], cy = (cell / d.nc[0]) % d.nc[1];
+  const int cz = cell / (d.nc[0] * d.nc[1]);
   d.xrel[k] = make_float4((float)(p[0] - cx * d.cellSize[0]), (float)(p[1] - cy * d.cellSize[1]),
-                          (float)(p[2] - cz * d.cellSize[2]), 0.f);
+                          (float)(p[2] - cz * d.cellSize[2]), __int_as_float(cx));
+  const int64_t off = id - d.idMin;
+  if (off < 0 || off >= d.idSpan)
+    atomicOr(d.err, kErrIdRange);
+  else
+    d.id2idx[off] = k;
 }
 
-__global__ void k_id_map(DevView d) {
-  const ParticleArrays a = d.pa[0];
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= d.n) return;
-  int64_t off = a.id[k] - d.idMin;
-  if (off < 0 || off >= d.idSpan) {
-    atomicOr(d.err, kErrIdRange);
-    return;
+// The last block to get here swaps the two copies of the arrays: every block has read their
+// pointers by then.
+__device__ __forceinline__ void swap_when_last(const DevView& d, const RebuildScratch& s,
+                                               const ParticleArrays& src,
+                                               const ParticleArrays& dst) {
+  __syncthreads();
+  if (threadIdx.x == 0 && atomicAdd(s.ticket, 1u) == gridDim.x - 1) {
+    *s.ticket = 0u;
+    d.pa[0] = dst;
+    d.pa[1] = src;
   }
-  d.id2idx[off] = k;
+}
+
+// Sorts the cells of a block: LANES lanes a cell (a quarter warp where cells hold few
+// particles) rank its particles by their keys in shared memory.  MOVE: the block's threads
+// then take its rows, a contiguous run, one each, and move them: one launch in place of an
+// in-cell sort, a gather, an id map and a swap, which is what a re-sort of a small system
+// costs (7.5 us for 32,768 particles, 18 as four kernels).  Its registers and the sort's
+// barrier leave a third of the threads in flight that a plain gather has, so large systems
+// (kMoveApart) write the order and move in a kernel of its own (100 us fused, 82 apart at a
+// million particles).  A cell's serial insertion sort by one lane took 115 us at 2,028
+// particles in 16 large cells, the ranking 8.
+constexpr int kSortThreads = 256;
+constexpr int kSortKeys = 1024;  // particles of a block ranked in shared memory
+constexpr int kMoveApart = 150000;
+
+template <int LANES, bool MOVE>
+__global__ void __launch_bounds__(kSortThreads) k_sort_cells(DevView d, RebuildScratch s) {
+  constexpr int kCells = kSortThreads / LANES;
+  __shared__ uint64_t s_key[kSortKeys];
+  __shared__ int s_ord[kSortKeys];
+  const ParticleArrays src = d.pa[0], dst = d.pa[1];
+  const int w = threadIdx.x / LANES, lane = threadIdx.x % LANES;
+  const int c0 = blockIdx.x * kCells, c = c0 + w;
+  const int first = d.cellStart[c0], rows = d.cellStart[min(c0 + kCells, d.ncells)] - first;
+  const int b = c < d.ncells ? d.cellStart[c] - first : 0;
+  const int n = c < d.ncells ? d.cellStart[c + 1] - first - b : 0;
+  const int cc[3] = {c % d.nc[0], (c / d.nc[0]) % d.nc[1], c / (d.nc[0] * d.nc[1])};
+  const bool fits = rows <= kSortKeys;
+  int* const perm = s.perm + first;
+  if (fits) {
+    for (int q = lane; q < n; q += LANES) s_key[b + q] = in_cell_key(d, src, perm[b + q], cc);
+    __syncwarp();
+    for (int q = lane; q < n; q += LANES) {
+      const uint64_t key = s_key[b + q];
+      int rank = 0;
+      for (int m = 0; m < n; ++m) rank += s_key[b + m] < key;
+      s_ord[b + rank] = perm[b + q];
+    }
+  } else if (lane == 0) {  // cells this full are sorted by insertion
+    for (int k = b + 1; k < b + n; ++k) {
+      const int v = perm[k];
+      const uint64_t key = in_cell_key(d, src, v, cc);
+      int m = k - 1;
+      while (m >= b && in_cell_key(d, src, perm[m], cc) > key) {
+        perm[m + 1] = perm[m];
+        --m;
+      }
+      perm[m + 1] = v;
+    }
+  }
+  __syncthreads();
+  if (MOVE) {
+    for (int q = threadIdx.x; q < rows; q += kSortThreads)
+      move_row(d, s, src, dst, fits ? s_ord[q] : perm[q], first + q);
+    swap_when_last(d, s, src, dst);
+  } else if (fits) {
+    for (int q = threadIdx.x; q < rows; q += kSortThreads) perm[q] = s_ord[q];
+  }
+}
+
+__global__ void __launch_bounds__(kBlock, 5) k_move(DevView d, RebuildScratch s) {
+  const ParticleArrays src = d.pa[0], dst = d.pa[1];
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < d.n) move_row(d, s, src, dst, s.perm[k], k);
+  swap_when_last(d, s, src, dst);
 }
 
 __global__ void k_posq(DevView d) {
@@ -314,31 +350,21 @@ __global__ void k_xrel(DevView d) {
   const int cx = cell % d.nc[0], cy = (cell / d.nc[0]) % d.nc[1], cz = cell / (d.nc[0] * d.nc[1]);
   d.xrel[k] = make_float4((float)(a.x[k] - cx * d.cellSize[0]),
                           (float)(a.x[(size_t)d.cap + k] - cy * d.cellSize[1]),
-                          (float)(a.x[2 * (size_t)d.cap + k] - cz * d.cellSize[2]), 0.f);
+                          (float)(a.x[2 * (size_t)d.cap + k] - cz * d.cellSize[2]),
+                          __int_as_float(cx));
 }
 
 // ---- Verlet list -------------------------------------------------------------------
 
-// ---- Verlet build, particle-per-lane form ------------------------------------------
-// One warp per cell and group of up to 32 of its particles; lane l holds particle g + l.
-// The candidates of each stencil row (the row's three x-cells) are staged 32 at a time
-// ("chunk") in shared memory, shifted into the cell's frame, and every lane tests all
-// of them against its particle, two candidates per packed f32x2 operation.  A lane
-// appends its partners to its own staging row and writes every full block of 8 to the
-// list with two 16-byte stores, so the list is written in whole sectors.  Candidates
-// are tested in FP32 on cell-relative coordinates; those within the relative 2e-5 band
+// Both forms of the build test the candidates of a run of particles in FP32 on coordinates
+// relative to a cell, staged in shared memory ("chunks"), two candidates per packed f32x2
+// operation, every lane against its own particle.  Candidates within the relative 2e-5 band
 // around (rc + skin)^2 are decided, after the chunk's other partners, by the reference's
 // FP64 arithmetic (exact_pair_test: d = p1 - (p2 + ghost shift), ((dx dx + dy dy) + dz dz),
 // Particle.hpp:93-98, DomainDecomposition.cpp:1347-1391).  The pair set is therefore the
-// reference's (VerletList.cpp:274-450), and each list is in a fixed order.
-constexpr int kBuildWarps = 4;
+// reference's (VerletList.cpp:274-450), and each list is in a fixed order.  Lists are written
+// in whole 32-byte sectors.
 constexpr int kStageLd = 44;  // staging row: <= 7 carried + <= 32 appended; 11 x 16 B
-
-struct BuildChunk {
-  float x[32], y[32], z[32];
-  int j[32];
-  int64_t id[32];
-};
 
 // Fast tests of one chunk (nv valid candidates) against the lane's particle.  Returns
 // whether any candidate came near the cutoff (a superset of the borderline band).
@@ -403,130 +429,6 @@ __device__ __forceinline__ void stage_flush(int* __restrict__ srow, int& pend, i
   pend = rem;
 }
 
-template <bool EXCL>
-__global__ void __launch_bounds__(kBuildWarps * 32) k_build_nl_lane(DevView d, double cutsq) {
-  const ParticleArrays a = d.pa[0];
-  __shared__ __align__(16) int s_stage[kBuildWarps][32 * kStageLd];
-  __shared__ __align__(16) BuildChunk s_chunk[kBuildWarps];
-  __shared__ int s_row[kBuildWarps][9][6];  // st0, ct0, st1, ct1, st2, ct2
-  const int wib = threadIdx.x >> 5;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (warp >= d.ncells) return;
-  const int c = warp;
-  const int cx = c % d.nc[0], cy = (c / d.nc[0]) % d.nc[1], cz = c / (d.nc[0] * d.nc[1]);
-  const int s0 = d.cellStart[c], s1 = d.cellStart[c + 1];
-  if (s0 == s1) return;
-  const float lo = (float)(cutsq * (1.0 - 2e-5)), hi = (float)(cutsq * (1.0 + 2e-5));
-  const float mid = (float)cutsq, hw = (float)(cutsq * 3e-5);
-  const unsigned long long mid2 = f2_pack(mid, mid);
-  const float hx = (float)d.cellSize[0], hy = (float)d.cellSize[1], hz = (float)d.cellSize[2];
-  const float4* __restrict__ xr = d.xrel;
-  const int K = d.K;
-  const size_t cap = d.cap;
-  int* __restrict__ nl = d.nl;
-  BuildChunk& ch = s_chunk[wib];
-  int* __restrict__ srow = &s_stage[wib][lane * kStageLd];
-  const int cxm = cx == 0 ? d.nc[0] - 1 : cx - 1;
-  const int cxp = cx == d.nc[0] - 1 ? 0 : cx + 1;
-  if (lane < 9) {
-    const int oz = lane / 3 - 1, oy = lane % 3 - 1;
-    int ncy = cy + oy, ncz = cz + oz;
-    ncy += ncy < 0 ? d.nc[1] : (ncy >= d.nc[1] ? -d.nc[1] : 0);
-    ncz += ncz < 0 ? d.nc[2] : (ncz >= d.nc[2] ? -d.nc[2] : 0);
-    const int rb = d.nc[0] * (ncy + d.nc[1] * ncz);
-    const int st0 = d.cellStart[rb + cxm], st1 = d.cellStart[rb + cx], st2 = d.cellStart[rb + cxp];
-    s_row[wib][lane][0] = st0;
-    s_row[wib][lane][1] = d.cellStart[rb + cxm + 1] - st0;
-    s_row[wib][lane][2] = st1;
-    s_row[wib][lane][3] = d.cellStart[rb + cx + 1] - st1;
-    s_row[wib][lane][4] = st2;
-    s_row[wib][lane][5] = d.cellStart[rb + cxp + 1] - st2;
-  }
-  __syncwarp();
-  for (int g = s0; g < s1; g += 32) {
-    const int ni = min(32, s1 - g);
-    const bool own = lane < ni;
-    const int i = own ? g + lane : g;
-    // padding lanes sit at +1e18 and invalid candidates at -1e18: no pair among them
-    // comes near the cutoff, and no square overflows FP32
-    const float4 ri = own ? xr[i] : make_float4(1e18f, 1e18f, 1e18f, 0.f);
-    const unsigned long long xi2 = f2_pack(ri.x, ri.x), yi2 = f2_pack(ri.y, ri.y);
-    const unsigned long long zi2 = f2_pack(ri.z, ri.z);
-    const int64_t idi = (EXCL && own) ? a.id[i] : -3;
-    int pend = 0, blk = 0;
-    for (int rr = 0; rr < 9; ++rr) {
-      const int oz = rr / 3 - 1, oy = rr % 3 - 1;
-      const int st0 = s_row[wib][rr][0], ct0 = s_row[wib][rr][1];
-      const int st1 = s_row[wib][rr][2], ct1 = s_row[wib][rr][3];
-      const int st2 = s_row[wib][rr][4], ct2 = s_row[wib][rr][5];
-      const int nrow = ct0 + ct1 + ct2;
-      for (int cb = 0; cb < nrow; cb += 32) {
-        const int nv = min(32, nrow - cb);
-        {
-          const int t = cb + lane;
-          const bool validj = t < nrow;
-          const int seg = t < ct0 ? 0 : (t < ct0 + ct1 ? 1 : 2);
-          const int j = !validj ? -1
-                                : (seg == 0 ? st0 + t : (seg == 1 ? st1 + t - ct0 : st2 + t - ct0 - ct1));
-          float4 rj = validj ? xr[j] : make_float4(-1e18f, -1e18f, -1e18f, 0.f);
-          ch.x[lane] = rj.x + (seg - 1) * hx;
-          ch.y[lane] = rj.y + oy * hy;
-          ch.z[lane] = rj.z + oz * hz;
-          ch.j[lane] = j;
-          if (EXCL) ch.id[lane] = validj ? a.id[j] : -2;
-        }
-        __syncwarp();
-        const bool band =
-            rr == 4 ? chunk_scan<true, EXCL>(d, ch, nv, xi2, yi2, zi2, i, idi, lo, mid2, hw, srow, pend)
-                    : chunk_scan<false, EXCL>(d, ch, nv, xi2, yi2, zi2, i, idi, lo, mid2, hw, srow,
-                                              pend);
-        if (__builtin_expect(__any_sync(0xffffffffu, band), 0) && own) {
-          // borderline candidates of this chunk: the reference's FP64 test decides
-          const int ncy = cy + oy, ncz = cz + oz;
-          const int wy = ncy < 0 ? -1 : (ncy >= d.nc[1] ? 1 : 0);
-          const int wz = ncz < 0 ? -1 : (ncz >= d.nc[2] ? 1 : 0);
-          for (int m = 0; m < nv; ++m) {
-            const unsigned long long dx = f2_sub(xi2, f2_pack(ch.x[m], ch.x[m]));
-            const unsigned long long dy = f2_sub(yi2, f2_pack(ch.y[m], ch.y[m]));
-            const unsigned long long dz = f2_sub(zi2, f2_pack(ch.z[m], ch.z[m]));
-            const float r2 = f2_lo(f2_fma(dz, dz, f2_fma(dy, dy, f2_mul(dx, dx))));
-            const int j = ch.j[m];
-            if (!(r2 >= lo && r2 <= hi) || j == i) continue;
-            const int t = cb + m;
-            const int seg = t < ct0 ? 0 : (t < ct0 + ct1 ? 1 : 2);
-            const int ox = seg - 1;
-            const int wx = seg == 0 ? (cx == 0 ? -1 : 0) : (seg == 2 ? (cx == d.nc[0] - 1 ? 1 : 0) : 0);
-            const bool fwd = oz > 0 || (oz == 0 && (oy > 0 || (oy == 0 && ox > 0)));
-            bool in = exact_pair_test(a.x, d.cap, i, j, fwd, wx * d.L[0], wy * d.L[1], wz * d.L[2],
-                                      cutsq);
-            if (EXCL && in && is_excluded(d, idi, ch.id[m])) in = false;
-            if (in) srow[pend++] = j;
-          }
-        }
-        stage_flush(srow, pend, blk, nl, i, cap, K >> 3);
-        __syncwarp();
-      }
-    }
-    const int total = blk * 8 + pend;
-    if (own) {
-      if (total > K) atomicOr(d.err, kErrNlOverflow);
-      d.nn[i] = min(total, K);
-      // pad to a multiple of 8 with the particle itself (r^2 = 0, masked by the force
-      // kernels) so that batches of 8 need no bounds checks; K is a multiple of 8
-      if (pend > 0) {
-        for (int k = pend; k < 8; ++k) srow[k] = i;
-        pend = 8;
-        stage_flush(srow, pend, blk, nl, i, cap, K >> 3);
-      }
-    }
-    const int wmax = __reduce_max_sync(0xffffffffu, own ? total : 0);
-    if (lane == 0 && wmax > 0) atomicMax(&d.ctr->nnMax, wmax);
-    __syncwarp();
-  }
-}
-
-
 // ---- Verlet build, run form ---------------------------------------------------------
 // One warp per 32 consecutive sorted particles, split where they change row of cells
 // (cy, cz); lane l holds particle g + l.  A group spans the x-cells ca..cb of one row; its
@@ -534,14 +436,11 @@ __global__ void __launch_bounds__(kBuildWarps * 32) k_build_nl_lane(DevView d, d
 // staged in the frame of cell (ca, cy, cz).  A candidate farther than the cutoff from the
 // bounding box of the group's particles cannot be a partner of any of them and is dropped
 // before it takes a slot of a chunk (ballot + prefix count), so the 32 lanes test only
-// survivors and no lane idles for lack of particles.  Tests, the band decided in FP64
-// and the staging of the list are those of the per-cell form.
-// Used for lists built right after the particles were binned at their current positions
-// in cells whose edges all exceed the list cutoff by 0.1 %: a particle's partners then
-// all lie in its 27 neighbour cells, and a candidate from a farther cell (a group spans
-// several x-cells) neither passes the test nor comes near the cutoff.  Grids with fewer
-// than 3 cells in a dimension, and lists rebuilt on cells of an earlier re-sort, use the
-// per-cell form.
+// survivors and no lane idles for lack of particles.
+// A candidate of a farther cell (a group spans several x-cells) neither passes the test nor
+// comes near the cutoff where the particles were binned at their current positions in cells
+// whose edges all exceed the list cutoff by 0.1 %; elsewhere (STALE) each particle's own
+// neighbour cells are enforced.
 constexpr int kRunWarps = 4;
 // x-cells a group may span: its candidate x-cells ca-h .. cb+h number at most 32
 
@@ -746,6 +645,360 @@ __global__ void __launch_bounds__(kRunWarps * 32) k_build_nl_run(DevView d, doub
     const int wmax = __reduce_max_sync(full, own ? total : 0);
     if (lane == 0 && wmax > 0) atomicMax(&d.ctr->nnMax, wmax);
     __syncwarp();
+  }
+}
+
+// ---- Verlet build, block form --------------------------------------------------------
+// The run form with four warps on one run of 32 particles: lane l of every warp holds
+// particle g + l, and the (2h+1)^2 rows of candidate cells are shared out among the warps
+// (block_row_owner).  A row's candidates are contiguous in the sorted order but for the
+// periodic wrap, so a warp streams them without a search and loads the next 32 while it tests
+// the last; it compacts the survivors of the bounding-box test over all its rows before it
+// scans them, keeps its partners in its own stage (transposed: entry-major, no bank conflicts)
+// and the block writes the lists once, in whole blocks of 8.
+// A warp alone spends about 7 cycles an instruction on this work, so a run handled by one
+// warp lasts 60 us however few particles there are.  Measured, run form against this one:
+// 62 / 20 us at 2,028 particles, 64 / 33 at 32,768, 157 / 137 at 241,133, 2.03 / 1.97 ms at
+// 4,096,000 (issue bound in both: about 400 instructions a particle), 49 / 24 at the
+// 40,000-bead melt.
+constexpr int kBlockW = 4;          // warps a run
+// Particles up to which two blocks share a run (SPLIT; one block a run: 36 us at 32,768, two:
+// 33; at 241,133 137 and 142, at 4,096,000 1.97 and 2.17 ms).
+constexpr int kBuildSplit = 100000;
+constexpr int kBlockListMax = 192;  // list capacity up to which the warps' shares fit the stages
+
+// Warp that takes row rr of the (2h+1)^2 rows, and its stage in entries.  One cell layer: the
+// centre row, with 29 of an LJ particle's 78 partners on average and 46 at most (counted on
+// 262,144 particles; about 60 where few cells make each a third wider), alone; opposite face
+// rows together (19, at most 37: a particle near one is far from the other); the four corner
+// rows together (10, at most 30).  With 6 blocks an SM, 240 entries a lane fill its shared
+// memory.
+__device__ __forceinline__ int block_row_owner(int rr, int h) {
+  return h > 1 ? rr % kBlockW : (int)((0x313202313ull >> (4 * rr)) & 15ull);
+}
+__host__ __device__ constexpr int block_stage_start(int w) {
+  return w == 0 ? 0 : (w == 1 ? 76 : (w == 2 ? 134 : (w == 3 ? 192 : 240)));
+}
+
+struct BlockWarp {
+  ulonglong2 a[32], b[32];  // candidate pairs: x0 x1, y0 y1; z0 z1, j0 j1
+  int code[64];             // x-cell relative to ca << 8 | row of cells
+};
+
+// Appends j at shared address `at` when r2 < lo (and j is not the particle itself): the store
+// is unconditional, only the advance is predicated, so a candidate costs three instructions
+// and no branch; a slot behind the last entry holds the last candidate that was no partner.
+template <bool SELF>
+__device__ __forceinline__ void stage_append(uint32_t& at, int j, float r2, float lo, int ip) {
+  if (SELF)
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.s32 q, %1, %4;\n\tsetp.lt.and.f32 p, %2, %3, q;\n\t"
+        "st.shared.b32 [%0], %1;\n\t@p add.u32 %0, %0, 128;\n\t}"
+        : "+r"(at)
+        : "r"(j), "f"(r2), "f"(lo), "r"(ip)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.lt.f32 p, %2, %3;\n\t"
+        "st.shared.b32 [%0], %1;\n\t@p add.u32 %0, %0, 128;\n\t}"
+        : "+r"(at)
+        : "r"(j), "f"(r2), "f"(lo)
+        : "memory");
+}
+
+// SPLIT: a run that changes row of cells is shared by two blocks, one for the first of its
+// groups, one (in the second half of the grid) for the others.  Where all blocks are resident
+// at once the kernel lasts as long as its slowest block, and a block of two groups takes twice
+// the time of one; a large grid only pays for the extra blocks.
+template <bool EXCL, bool STENCIL, bool SPLIT>
+__global__ void __launch_bounds__(32 * kBlockW, 6) k_build_block(DevView d, double cutsq) {
+  const ParticleArrays a = d.pa[0];
+  constexpr int W = kBlockW;
+  __shared__ __align__(16) BlockWarp s_w[W];
+  __shared__ int s_stage[block_stage_start(W) * 32];
+  __shared__ int s_cnt[W][32];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool second = SPLIT && blockIdx.x >= gridDim.x / 2;
+  const int g = (SPLIT ? (int)(blockIdx.x - (second ? gridDim.x / 2 : 0)) : (int)blockIdx.x) * 32;
+  const unsigned full = 0xffffffffu;
+  const float lo = (float)(cutsq * (1.0 - 2e-5)), hi = (float)(cutsq * (1.0 + 2e-5));
+  const float mid = (float)cutsq, hw = (float)(cutsq * 3e-5);
+  const float keepsq = (float)(cutsq * (1.0 + 1e-4));
+  const unsigned long long mid2 = f2_pack(mid, mid);
+  const float hx = (float)d.cellSize[0], hy = (float)d.cellSize[1], hz = (float)d.cellSize[2];
+  const int nx = d.nc[0], ny = d.nc[1], nz = d.nc[2];
+  const int h = d.hci, sw = 2 * h + 1;
+  const float4* __restrict__ xr = d.xrel;
+  BlockWarp& sm = s_w[w];
+  float* const sa = reinterpret_cast<float*>(sm.a);
+  float* const sb = reinterpret_cast<float*>(sm.b);
+  const int ip = g + lane;
+  const bool valid = ip < d.n;
+  const float4 me = valid ? xr[ip] : make_float4(0.f, 0.f, 0.f, 0.f);
+  const int mcx = __float_as_int(me.w);
+  const int mrow = valid ? d.pcell[ip] - mcx : 0;  // first cell of the particle's row of cells
+  const int64_t idi = (EXCL && valid) ? a.id[ip] : -3;
+  const bool mayself = h > 1 || w == 0;  // the warp's rows hold the particles themselves
+  // shared addresses of the lane's stage, 128 bytes an entry: first, next, and the last next
+  // that leaves room for the 8 candidates tested between two checks
+  const uint32_t st0 =
+      (uint32_t)__cvta_generic_to_shared(s_stage + 32 * block_stage_start(w) + lane);
+  const uint32_t stLast = st0 + 128u * (block_stage_start(w + 1) - block_stage_start(w) - 9);
+  uint32_t at = st0;
+  bool over = false;
+  unsigned todo = __ballot_sync(full, valid), mine = todo;
+  bool skip = second;  // the first group is the other block's
+  while (todo) {
+    const int leader = __ffs(todo) - 1;
+    const int row = __shfl_sync(full, mrow, leader);
+    const int ca = __shfl_sync(full, mcx, leader);
+    const unsigned grp =
+        __ballot_sync(full, ((todo >> lane) & 1u) && mrow == row && mcx - ca <= (1 << 20));
+    todo &= ~grp;
+    if (SPLIT) {
+      if (skip) {
+        skip = false;
+        mine &= ~grp;
+        continue;
+      }
+      if (!second) {
+        todo = 0u;
+        mine = grp;
+      }
+    }
+    const bool own = (grp >> lane) & 1u;
+    const int cb = __shfl_sync(full, mcx, 31 - __clz(grp));
+    const int rowOf = row / nx, cz = rowOf / ny, cy = rowOf - cz * ny;
+    const int rel = mcx - ca;
+    // the lane's particle in the frame of cell (ca, cy, cz); lanes outside the group far away
+    const float fx = own ? me.x + (float)rel * hx : 1e18f;
+    const float fy = own ? me.y : 1e18f, fz = own ? me.z : 1e18f;
+    const float bxl = warp_fmin(own ? fx : 3e38f), bxh = warp_fmax(own ? fx : -3e38f);
+    const float byl = warp_fmin(own ? fy : 3e38f), byh = warp_fmax(own ? fy : -3e38f);
+    const float bzl = warp_fmin(own ? fz : 3e38f), bzh = warp_fmax(own ? fz : -3e38f);
+    const unsigned long long xi2 = f2_pack(fx, fx), yi2 = f2_pack(fy, fy), zi2 = f2_pack(fz, fz);
+
+    // tests the first nv candidates of the chunk (filled up to a multiple of 8) against the
+    // lane's particle
+    auto scan = [&](int nv, auto self) {
+      float near = 3e38f;  // smallest |r^2 - cutoff^2|
+      for (int m0 = 0; m0 < nv; m0 += 8) {
+        // all loads before the first append: a store to the stage keeps later loads behind it
+        ulonglong2 A[4], B[4];
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+          A[p] = sm.a[(m0 >> 1) + p];
+          B[p] = sm.b[(m0 >> 1) + p];
+        }
+        unsigned long long r2p[4];
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+          const unsigned long long dx = f2_sub(xi2, A[p].x), dy = f2_sub(yi2, A[p].y);
+          const unsigned long long dz = f2_sub(zi2, B[p].x);
+          r2p[p] = f2_fma(dz, dz, f2_fma(dy, dy, f2_mul(dx, dx)));
+          const unsigned long long t = f2_sub(r2p[p], mid2);
+          near = fminf(fminf(near, fabsf(f2_lo(t))), fabsf(f2_hi(t)));
+        }
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+          const unsigned long long r2 = r2p[p];
+          const int ja = (int)(unsigned)B[p].y, jb = (int)(B[p].y >> 32);
+          if constexpr (!EXCL && !STENCIL) {
+            stage_append<decltype(self)::value>(at, ja, f2_lo(r2), lo, ip);
+            stage_append<decltype(self)::value>(at, jb, f2_hi(r2), lo, ip);
+          } else {
+            bool ina = f2_lo(r2) < lo && ja != ip, inb = f2_hi(r2) < lo && jb != ip;
+            if (STENCIL) {
+              const int2 c = *reinterpret_cast<const int2*>(&sm.code[m0 + 2 * p]);
+              ina &= (unsigned)((c.x >> 8) - rel + h) <= (unsigned)(2 * h);
+              inb &= (unsigned)((c.y >> 8) - rel + h) <= (unsigned)(2 * h);
+            }
+            if (EXCL) {
+              if (ina && is_excluded(d, idi, a.id[ja])) ina = false;
+              if (inb && is_excluded(d, idi, a.id[jb])) inb = false;
+            }
+            stage_append<false>(at, ja, ina ? 0.f : 1.f, 0.5f, ip);
+            stage_append<false>(at, jb, inb ? 0.f : 1.f, 0.5f, ip);
+          }
+        }
+        over |= at > stLast;
+        at = min(at, stLast);
+      }
+      if (__builtin_expect(__any_sync(full, near <= hw), 0) && own && near <= hw) {
+        // borderline candidates of this chunk: the reference's FP64 test decides
+        for (int m = 0; m < nv; ++m) {
+          const int q = 4 * (m >> 1) + (m & 1);
+          const float x = sa[q], y = sa[q + 2], z = sb[q];
+          const unsigned long long dx = f2_sub(xi2, f2_pack(x, x));
+          const unsigned long long dy = f2_sub(yi2, f2_pack(y, y));
+          const unsigned long long dz = f2_sub(zi2, f2_pack(z, z));
+          const float r2 = f2_lo(f2_fma(dz, dz, f2_fma(dy, dy, f2_mul(dx, dx))));
+          const int j = __float_as_int(sb[q + 2]), code = sm.code[m];
+          if (!(r2 >= lo && r2 <= hi) || j == ip) continue;
+          const int oz = (code & 255) / sw - h, oy = (code & 255) % sw - h;
+          const int xu = ca + (code >> 8);  // the candidate's x-cell, unwrapped
+          const int ox = xu - mcx;
+          if (ox < -h || ox > h) continue;  // not a neighbour cell of this particle
+          const int wx = xu < 0 ? -1 : (xu >= nx ? 1 : 0);
+          const int wy = cy + oy < 0 ? -1 : (cy + oy >= ny ? 1 : 0);
+          const int wz = cz + oz < 0 ? -1 : (cz + oz >= nz ? 1 : 0);
+          const bool fwd = oz > 0 || (oz == 0 && (oy > 0 || (oy == 0 && ox > 0)));
+          bool in = exact_pair_test(a.x, d.cap, ip, j, fwd, wx * d.L[0], wy * d.L[1],
+                                    wz * d.L[2], cutsq);
+          if (EXCL && in && is_excluded(d, idi, a.id[j])) in = false;
+          if (in) {
+            if (at < stLast)
+              stage_append<false>(at, j, 0.f, 1.f, ip);
+            else
+              over = true;
+          }
+        }
+      }
+    };
+
+    // Segments: the candidates of a row of cells below, inside and above the box, each a
+    // contiguous run of sorted particles; one lane looks up each.
+    int fill = 0;
+    const int nseg = 3 * sw * sw;
+    for (int seg0 = 0; seg0 < nseg; seg0 += 32) {
+      const int sg = seg0 + lane, rr = sg / 3, p = sg % 3 - 1;
+      int js = 0, je = 0, code = 0;  // code: x shift of the frame, row, oz + h, oy + h
+      if (sg < nseg) {
+        const int oz1 = h == 1 ? rr / 3 : rr / sw, oy1 = rr - oz1 * sw;
+        const int xs = max(ca - h, p * nx), xe = min(cb + h, p * nx + nx - 1);
+        if (block_row_owner(rr, h) == w && xs <= xe) {
+          const int ncy = cy + oy1 - h, ncz = cz + oz1 - h;
+          const int wcy = ncy < 0 ? ncy + ny : (ncy >= ny ? ncy - ny : ncy);
+          const int wcz = ncz < 0 ? ncz + nz : (ncz >= nz ? ncz - nz : ncz);
+          const int rb = nx * (wcy + ny * wcz) - p * nx;
+          js = d.cellStart[rb + xs];
+          je = d.cellStart[rb + xe + 1];
+          code = (p + 1) << 24 | rr << 16 | oz1 << 8 | oy1;
+        }
+      }
+      unsigned segs = __ballot_sync(full, js < je);
+      // the next round's candidates are loaded before this round's are filtered and scanned
+      int nj = 0, ne = 0, nbase = 0, nrr = 0;  // next round: first, end, x shift, row
+      float nofy = 0.f, nofz = 0.f;
+      float4 nxt = make_float4(0.f, 0.f, 0.f, 0.f);
+      auto load_round = [&](bool advance) {
+        if (advance) {
+          nj = ne = 0;
+          if (segs) {
+            const int src = __ffs(segs) - 1;
+            segs &= segs - 1;
+            nj = __shfl_sync(full, js, src);
+            ne = __shfl_sync(full, je, src);
+            const int c = __shfl_sync(full, code, src);
+            nbase = ((c >> 24) - 1) * nx - ca;
+            nrr = (c >> 16) & 255;
+            nofz = (float)(((c >> 8) & 255) - h) * hz;
+            nofy = (float)((c & 255) - h) * hy;
+          }
+        }
+        if (nj + lane < ne) nxt = xr[nj + lane];
+      };
+      load_round(true);
+      while (nj < ne) {
+        const int cj = nj, ce = ne, cbase = nbase, crr = nrr;
+        const float ofy = nofy, ofz = nofz;
+        const float4 rj = nxt;
+        nj += 32;
+        load_round(nj >= ne);
+        const int j = cj + lane;
+        const int xo = __float_as_int(rj.w) + cbase;  // x-cell relative to ca
+        const float cx = rj.x + (float)xo * hx, cyf = rj.y + ofy, czf = rj.z + ofz;
+        const float ex = fmaxf(0.f, fmaxf(bxl - cx, cx - bxh));
+        const float ey = fmaxf(0.f, fmaxf(byl - cyf, cyf - byh));
+        const float ez = fmaxf(0.f, fmaxf(bzl - czf, czf - bzh));
+        const bool keep = j < ce && fmaf(ez, ez, fmaf(ey, ey, ex * ex)) <= keepsq;
+        const unsigned km = __ballot_sync(full, keep);
+        if (keep) {
+          const int pos = fill + __popc(km & ((1u << lane) - 1u));
+          const int q = 4 * (pos >> 1) + (pos & 1);
+          sa[q] = cx;
+          sa[q + 2] = cyf;
+          sb[q] = czf;
+          sb[q + 2] = __int_as_float(j);
+          sm.code[pos] = xo * 256 + crr;
+        }
+        fill += __popc(km);
+        if (fill >= 32) {
+          __syncwarp();
+          if (mayself)
+            scan(32, std::true_type{});
+          else
+            scan(32, std::false_type{});
+          __syncwarp();
+          // slots 32 .. fill-1 move to the front
+          if (lane < (fill - 31) >> 1) {
+            sm.a[lane] = sm.a[16 + lane];
+            sm.b[lane] = sm.b[16 + lane];
+          }
+          if (lane < fill - 32) sm.code[lane] = sm.code[32 + lane];
+          fill -= 32;
+          __syncwarp();
+        }
+      }
+    }
+    if (fill > 0) {
+      // far-away candidates fill the last 8
+      const int pos = fill + lane;
+      if (pos < ((fill + 7) & ~7)) {
+        const int q = 4 * (pos >> 1) + (pos & 1);
+        sa[q] = sa[q + 2] = sb[q] = -1e18f;
+        sb[q + 2] = __int_as_float(-1);
+        sm.code[pos] = 0;
+      }
+      __syncwarp();
+      if (mayself)
+        scan(fill, std::true_type{});
+      else
+        scan(fill, std::false_type{});
+      __syncwarp();
+    }
+  }
+  if (SPLIT && mine == 0u) return;  // the whole block: a run of one group
+  const bool write = (mine >> lane) & 1u;
+  s_cnt[w][lane] = (int)(at - st0) >> 7;
+  if (over) atomicOr(d.err, kErrNlOverflow);
+  __syncthreads();
+  // the lists: thread (w, lane) writes the blocks w, w + W, ... of particle g + lane
+  int pre[W + 1], base[W];  // base: where entry k of the list would lie in warp u's stage
+  pre[0] = 0;
+#pragma unroll
+  for (int u = 0; u < W; ++u) {
+    pre[u + 1] = pre[u] + s_cnt[u][lane];
+    base[u] = block_stage_start(u) - pre[u];
+  }
+  const int total = pre[W], K = d.K;
+  if (write) {
+    if (w == 0) {
+      d.nn[ip] = min(total, K);
+      if (total > K) atomicOr(d.err, kErrNlOverflow);
+    }
+    const int fit = min(total, K);
+    for (int b = w; 8 * b < fit; b += W) {
+      // padded to a multiple of 8 with the particle itself (r^2 = 0, masked by the force
+      // kernels) so that blocks of 8 need no bounds checks; K is a multiple of 8
+      int v[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const int k = 8 * b + e;
+        int at = base[0];
+#pragma unroll
+        for (int u = 1; u < W; ++u) at = k >= pre[u] ? base[u] : at;
+        v[e] = k < total ? s_stage[32 * (at + k) + lane] : ip;
+      }
+      int4* dst = reinterpret_cast<int4*>(d.nl + nl_index(8 * b, ip, d.cap));
+      dst[0] = make_int4(v[0], v[1], v[2], v[3]);
+      dst[1] = make_int4(v[4], v[5], v[6], v[7]);
+    }
+  }
+  if (w == 0) {
+    const int wmax = __reduce_max_sync(full, write ? total : 0);
+    if (lane == 0 && wmax > 0) atomicMax(&d.ctr->nnMax, wmax);
   }
 }
 
@@ -1141,17 +1394,6 @@ __global__ void k_decide_graph(DevCounters* c, double skinHalf, cudaGraphConditi
   const int f = decide_core(c, skinHalf);
   cudaGraphSetConditional(hIf, f ? 1u : 0u);
   cudaGraphSetConditional(hWhile, rem > 0 ? 1u : 0u);
-}
-
-__global__ void k_zero_i32(int32_t* p, int n) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) p[i] = 0;
-}
-
-__global__ void k_swap_arrays(ParticleArrays* pa) {
-  const ParticleArrays t = pa[0];
-  pa[0] = pa[1];
-  pa[1] = t;
 }
 
 // ---- observables -------------------------------------------------------------------
@@ -1833,28 +2075,33 @@ __global__ void __launch_bounds__(256) k_fma_probe(float* out, int iters) {
 // ---- launchers ---------------------------------------------------------------------
 
 void launch_fold_bin(const DevView& d, RebuildScratch& s, bool fold, cudaStream_t st) {
-  k_zero_i32<<<blocks_for(d.ncells), kBlock, 0, st>>>(s.cellCount, d.ncells);
   if (d.n > 0) k_fold_bin<<<blocks_for(d.n), kBlock, 0, st>>>(d, s, fold ? 1 : 0);
-}
-
-void launch_sort_cells(const DevView& d, RebuildScratch& s, cudaStream_t st) {
-  const int ntiles = (d.ncells + kScanTile - 1) / kScanTile;
-  k_scan_tiles<<<ntiles, kScanBlock, 0, st>>>(s.cellCount, d.ncells, s.tileSum);
-  k_scan_tile_sums<<<1, kScanBlock, 0, st>>>(s.tileSum, ntiles);
-  k_scan_apply<<<ntiles, kScanBlock, 0, st>>>(s.cellCount, d.ncells, s.tileSum, d.cellStart);
-  if (d.n > 0) k_scatter<<<blocks_for(d.n), kBlock, 0, st>>>(d, s);
-  k_sort_in_cell<<<blocks_for((long long)d.ncells * 32), kBlock, 0, st>>>(d, s);
 }
 
 int scan_tiles(int ncells) { return (ncells + kScanTile - 1) / kScanTile; }
 
-void launch_gather(const DevView& d, const RebuildScratch& s, cudaStream_t st) {
-  if (d.n > 0) k_gather<<<blocks_for(d.n), kBlock, 0, st>>>(d, s);
-  k_swap_arrays<<<1, 1, 0, st>>>(d.pa);
+// Cell starts, then the particles into their cells' rows of the other copy of the arrays
+// (swapped on the device).
+void launch_sort_cells(const DevView& d, RebuildScratch& s, cudaStream_t st) {
+  const int ntiles = scan_tiles(d.ncells);
+  if (ntiles > 1) k_scan_tiles<<<ntiles, kScanBlock, 0, st>>>(s.cellCount, d.ncells, s.tileSum);
+  k_scan_apply<<<ntiles, kScanBlock, 0, st>>>(s.cellCount, d.ncells, s.tileSum, d.cellStart);
+  if (d.n == 0) return;
+  k_scatter<<<blocks_for(d.n), kBlock, 0, st>>>(d, s);
+  // 8 lanes a cell up to 6 particles a cell on average
+  const bool few = d.n <= 6ll * d.ncells, move = d.n < kMoveApart;
+  const int nb = blocks_for(d.ncells, kSortThreads / (few ? 8 : 32));
+  if (few)
+    move ? k_sort_cells<8, true><<<nb, kSortThreads, 0, st>>>(d, s)
+         : k_sort_cells<8, false><<<nb, kSortThreads, 0, st>>>(d, s);
+  else
+    move ? k_sort_cells<32, true><<<nb, kSortThreads, 0, st>>>(d, s)
+         : k_sort_cells<32, false><<<nb, kSortThreads, 0, st>>>(d, s);
+  if (!move) k_move<<<blocks_for(d.n), kBlock, 0, st>>>(d, s);
 }
 
-void launch_id_map(const DevView& d, cudaStream_t st) {
-  if (d.n > 0) k_id_map<<<blocks_for(d.n), kBlock, 0, st>>>(d);
+int resort_launches(const DevView& d) {
+  return 4 + (scan_tiles(d.ncells) > 1 ? 1 : 0) + (d.n < kMoveApart ? 0 : 1);
 }
 
 void launch_xrel(const DevView& d, cudaStream_t st) {
@@ -1865,47 +2112,39 @@ void launch_posq(const DevView& d, cudaStream_t st) {
   if (d.n > 0) k_posq<<<blocks_for(d.n), kBlock, 0, st>>>(d);
 }
 
-// The run form needs cells binned at the current positions (fresh), at least 3 cells in
-// every dimension and cell edges 0.1 % above the list cutoff; ESPP_B200_BUILD=cell keeps
-// the per-cell form.
-bool run_build_ok(const DevView& d, double cutsq, bool fresh) {
-  static int env = -1;
-  if (env < 0) {
-    const char* e = getenv("ESPP_B200_BUILD");
-    env = (e && strcmp(e, "cell") == 0) ? 0 : 1;
-  }
-  if (!fresh || env == 0 || d.n == 0) return false;
-  const double rc = sqrt(cutsq) * (1.0 + 1e-3) / d.hci;
-  for (int k = 0; k < 3; ++k)
-    if (d.nc[k] < 2 * d.hci + 1 || d.cellSize[k] < rc) return false;
-  return true;
-}
-
+// Cells binned at the current positions (fresh) with edges 0.1 % above the list cutoff need
+// no check of a candidate's cell (see the run form); otherwise each particle's own neighbour
+// cells are enforced.  The block form's stages hold lists of up to kBlockListMax entries;
+// longer lists (a list that overflows is rebuilt with twice the capacity) take the run form,
+// which writes its lists as it goes.
 void launch_build_nl(const DevView& d, double cutsq, bool fresh, cudaStream_t st) {
-  if (run_build_ok(d, cutsq, fresh)) {
-    const int nb = blocks_for((long long)d.n, kRunWarps * 32);
-    if (d.exclStart)
-      k_build_nl_run<true, false><<<nb, kRunWarps * 32, 0, st>>>(d, cutsq);
-    else
-      k_build_nl_run<false, false><<<nb, kRunWarps * 32, 0, st>>>(d, cutsq);
-    return;
-  }
-  if (d.hci > 1) {
-    // the per-cell form reaches one cell; the run form with each particle's own
-    // neighbour cells enforced serves any cells (also cells of an earlier re-sort)
-    if (d.n == 0) return;
-    const int nb = blocks_for((long long)d.n, kRunWarps * 32);
-    if (d.exclStart)
-      k_build_nl_run<true, true><<<nb, kRunWarps * 32, 0, st>>>(d, cutsq);
-    else
-      k_build_nl_run<false, true><<<nb, kRunWarps * 32, 0, st>>>(d, cutsq);
-    return;
-  }
-  const int nb = blocks_for((long long)d.ncells * 32, kBuildWarps * 32);
-  if (d.exclStart)
-    k_build_nl_lane<true><<<nb, kBuildWarps * 32, 0, st>>>(d, cutsq);
+  if (d.n == 0) return;
+  const double rc = sqrt(cutsq) * (1.0 + 1e-3) / d.hci;
+  bool stencil = !fresh;
+  for (int k = 0; k < 3; ++k) stencil = stencil || d.cellSize[k] < rc;
+  const bool excl = d.exclStart != nullptr;
+#define ESPP_BUILD_CASE(KERNEL, NB, NT)                                    \
+  do {                                                                     \
+    if (excl)                                                              \
+      stencil ? KERNEL(true, true)<<<NB, NT, 0, st>>>(d, cutsq)            \
+              : KERNEL(true, false)<<<NB, NT, 0, st>>>(d, cutsq);          \
+    else                                                                   \
+      stencil ? KERNEL(false, true)<<<NB, NT, 0, st>>>(d, cutsq)           \
+              : KERNEL(false, false)<<<NB, NT, 0, st>>>(d, cutsq);         \
+  } while (0)
+#define ESPP_RUN(E, S) k_build_nl_run<E, S>
+#define ESPP_BLOCK(E, S) k_build_block<E, S, false>
+#define ESPP_BLOCK2(E, S) k_build_block<E, S, true>
+  if (d.K > kBlockListMax)
+    ESPP_BUILD_CASE(ESPP_RUN, blocks_for((long long)d.n, kRunWarps * 32), kRunWarps * 32);
+  else if (d.n < kBuildSplit)
+    ESPP_BUILD_CASE(ESPP_BLOCK2, 2 * blocks_for((long long)d.n, 32), 32 * kBlockW);
   else
-    k_build_nl_lane<false><<<nb, kBuildWarps * 32, 0, st>>>(d, cutsq);
+    ESPP_BUILD_CASE(ESPP_BLOCK, blocks_for((long long)d.n, 32), 32 * kBlockW);
+#undef ESPP_BUILD_CASE
+#undef ESPP_RUN
+#undef ESPP_BLOCK
+#undef ESPP_BLOCK2
 }
 
 template <int TPP, bool MIXED>
