@@ -165,6 +165,7 @@ struct espp_system {
   // Verlet list
   bool has_vl = false;
   double vl_cut = 0.0;
+  double listSkin = 0.0;  // skin of the last list build
   std::vector<std::pair<int64_t, int64_t>> vlExcl;
   int64_t builds = 0;
 
@@ -228,7 +229,7 @@ struct espp_system {
   IntegrateArgs ddArgs{};
   int capMode = ESPP_CAP_OFF;
   double cap3[3] = {0, 0, 0};
-  int tpp = 4;
+  int tpp = 0;  // threads per particle of the force pass; 0: chosen by size (force_tpp)
   double timers[10] = {0};
 
   // host id list (all particle ids, for the id map) and the largest type present
@@ -248,6 +249,17 @@ struct espp_system {
     b.nl = bnl;
     b.Kb = bKb;
     return b;
+  }
+
+  // Partners lie within the list cutoff and the drift since the build (skin / 2 a particle);
+  // the box has to be wide enough that such a difference is its own minimum image.  Not after
+  // positions were set from outside (a re-sort is pending).
+  double wrap_margin() const {
+    if (resortFlag) return 1e300;
+    const double m = vl_cut + 3.0 * std::max(skin, listSkin);
+    for (int k = 0; k < 3; ++k)
+      if (L[k] < 2.0 * m) return 1e300;
+    return m;
   }
 
   DevView view() const {
@@ -274,6 +286,7 @@ struct espp_system {
     d.nl = nl;
     d.nn = nn;
     d.K = K;
+    d.wrapMargin = wrap_margin();
     d.ffix = ffix;
     d.f64 = f64;
     d.ftot = ftot;
@@ -781,6 +794,7 @@ void build_list(espp_system* s) {
   if (!s->binned) bin(s, false);
   double cutVerlet = s->vl_cut + s->skin;
   double cutsq = cutVerlet * cutVerlet;
+  s->listSkin = s->skin;
   s->brickOn = brick_wanted(s) && s->n > 0;
   if (s->brickOn && !build_list_brick(s, cutsq)) {
     s->brickOn = false;
@@ -902,6 +916,18 @@ void ensure_mlp_scratch(espp_system* s) {
   s->mlpCap = s->cap;
 }
 
+// Threads per particle of the force pass: the caller's, else by size.
+int force_tpp(const espp_system* s) {
+  if (s->tpp > 0) return s->tpp;
+  // Lanes fill the GPU at small sizes and share their gathers' lines; at large ones each more
+  // lane leaves fewer entries a lane.  Force pass, 1 / 2 / 4 lanes, mixed: 9.1 / 7.1 / 6.8 us at
+  // 2,028 particles, 11.2 / 9.2 / 9.2 at 32,768, 40.6 / 37.9 / 39.9 at 241,133, 131 / 136 / 159
+  // at 1,009,091, 505 / 550 / 670 at 4,096,000.  Below, as many as one block an SM of the step
+  // kernel has room for.
+  const int four = s->precision == ESPP_PREC_MIXED ? 37000 : 23000;
+  return s->n >= 600000 ? 1 : (s->n >= four ? 2 : 4);
+}
+
 // Main pair + FENE kernel (list counts zeroed when no LJ pair is set), then the
 // tabulated pair and bond forces added to its output.
 void launch_all_forces(espp_system* s, cudaStream_t st) {
@@ -912,7 +938,7 @@ void launch_all_forces(espp_system* s, cudaStream_t st) {
     launch_forces_brick(d, mixed, s->fene, st);
   } else {
     if (!s->has_vl || !s->lj_any) dm.nn = s->nnZero;  // no LJ term: bonds only
-    launch_forces(dm, mixed, s->fene, s->tpp, st);
+    launch_forces(dm, mixed, s->fene, force_tpp(s), st);
   }
   if (!s->has_vl) d.tabNT = 0;
   launch_force_tab(d, mixed, st);
@@ -1033,7 +1059,7 @@ std::string graph_key(espp_system* s, const IntegrateArgs& a) {
   std::string k((const char*)&d, sizeof(d));
   k.append((const char*)&a, sizeof(a));
   k.append((const char*)&s->fene, sizeof(s->fene));
-  int extra[4] = {s->tpp, s->has_vl ? 1 : 0, s->lj_any ? 1 : 0, s->precision};
+  int extra[4] = {force_tpp(s), s->has_vl ? 1 : 0, s->lj_any ? 1 : 0, s->precision};
   k.append((const char*)extra, sizeof(extra));
   double sk = s->skin + s->vl_cut;
   k.append((const char*)&sk, sizeof(sk));
@@ -1300,6 +1326,7 @@ void graph_loop_done(espp_system* s, int64_t nsteps) {
   s->step += nsteps;
   s->nResorts = c.resorts;
   s->builds += c.resorts;
+  if (c.resorts) s->listSkin = s->skin;
   // kernels launched by the graph: decide + force + integrate per step, and fold/bin, scan
   // (1 or 2), scatter, sort, move (+ list) per re-sort
   s->phaseLaunches[kPhOther] += nsteps;
@@ -3222,7 +3249,7 @@ int espp_get_layout(espp_system* s, int32_t out[5]) {
     checked(s);
     if (!out) raise(ESPP_EINVAL, "null output pointer");
     out[0] = s->brickOn ? 1 : (s->brickBuildUsed ? 2 : 0);
-    out[1] = s->tpp;
+    out[1] = force_tpp(s);
     for (int k = 0; k < 3; ++k) out[2 + k] = (s->brickOn || s->brickBuildUsed) ? s->brickB[k] : 0;
   });
 }
@@ -3284,7 +3311,7 @@ int espp_autotune_layout(espp_system* s, double steps_per_build, int32_t best[5]
     if (ncand) *ncand = row;
     if (best) {
       best[0] = s->brickOn ? 1 : (s->brickBuildUsed ? 2 : 0);
-      best[1] = s->tpp;
+      best[1] = force_tpp(s);
       for (int k = 0; k < 3; ++k)
         best[2 + k] = (s->brickOn || s->brickBuildUsed) ? s->brickB[k] : 0;
     }

@@ -159,6 +159,8 @@ struct DevView {
   int32_t* nl;            // K * cap, blocks of 8: entry (k, i) at ((k/8)*cap + i)*8 + k%8
   int32_t* nn;            // neighbour count per particle
   int K;                  // neighbour capacity
+  double wrapMargin;      // a particle farther than this from every face of the box has no
+                          // partner across one
   long long* ffix;        // 3*cap pair+bond force, int64 2^-32 fixed point (mixed)
   double* f64;            // 3*cap pair+bond force (FP64 path)
   double* ftot;           // 3*cap total force after the aftCalcF extensions

@@ -1004,117 +1004,111 @@ __global__ void __launch_bounds__(32 * kBlockW, 6) k_build_block(DevView d, doub
 
 // ---- forces ------------------------------------------------------------------------
 
-// FP32 pair forces on box-wrapped int32 coordinates.  The minimum image is the 32-bit
-// wrap of the coordinate difference.  One thread per particle (TPP threads when >1),
-// FP32 sums along the list, results stored as int64 2^-32 fixed point; partial sums
-// of the TPP threads and the bond term are combined in int64, so the result does not
-// depend on the order in which they are added.
-template <int TPP, bool SINGLE, bool CAPPED, bool FENE>
-__global__ void __launch_bounds__(256) k_force_mixed(DevView d, FENEParams fp) {
+constexpr int kMixMB = 4;
+// Loads of arrays that other blocks write during the kernel (LIVE) go through the coherent
+// path, others through the read-only one.
+template <bool LIVE>
+__device__ __forceinline__ int4 ld_pos(const int4* p) {
+  if (!LIVE) return __ldg(p);
+  int4 v;
+  asm volatile("ld.global.v4.s32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(p)
+               : "memory");
+  return v;
+}
+template <bool LIVE>
+__device__ __forceinline__ double ld_pos(const double* p) {
+  if (!LIVE) return __ldg(p);
+  double v;
+  asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
+  return v;
+}
+
+// FP32 pair forces on box-wrapped int32 coordinates, T lanes a particle.  The minimum image
+// is the 32-bit wrap of the coordinate difference.  Two entries are evaluated at once in the
+// halves of packed f32x2 registers (20 instructions an entry, 31 scalar).  FP32 sums along
+// the list, the result in int64 2^-32 fixed point; the lanes' partial sums and the bond
+// terms are combined in int64, so the result does not depend on the order in which they are
+// added.  Every lane of the warp takes part (act: the lane has a particle).
+// Bound by the L1 data pipe: the 32 coordinates a warp gathers lie in 10 to 18 lines, 88 to 95 %
+// of the pipe's wavefronts at a million particles, issue 39 % (53 % scalar).  With ListShare
+// the lanes of a particle take adjacent entries, which share lines.  At 241,133 particles of
+// two types 59.0 us before and 46.1 now, at 32,768 11.1 and 8.1; 4,096,000 with one lane 505.
+template <int T, bool SINGLE, bool CAPPED, bool FENE, bool LIVE, class Share>
+__device__ __forceinline__ void particle_force_mixed(const DevView& d, const FENEParams& fp,
+                                                     const LJPairF* sP, const int4* posq, int i,
+                                                     int sub, bool act, const Share& share,
+                                                     long long (&F)[3]) {
   const ParticleArrays a = d.pa[0];
-  __shared__ LJPairF sP[kMaxTypes * kMaxTypes];
-  if (!SINGLE) {
-    for (int t = threadIdx.x; t < d.ntypes * d.ntypes; t += blockDim.x) sP[t] = d.ljf[t];
-    __syncthreads();
-  }
-  const int gt = blockIdx.x * blockDim.x + threadIdx.x;
-  const int i0 = gt / TPP;
-  const int sub = gt % TPP;
-  if (TPP == 1 && i0 >= d.n) return;
-  // with TPP > 1 every lane stays until the shuffles below
-  const bool act = i0 < d.n;
-  const int i = act ? i0 : 0;
-  const int4 pi = d.posq[i];
-  const float ux = d.fixUnit[0], uy = d.fixUnit[1], uz = d.fixUnit[2];
-  const int cnt = act ? d.nn[i] : 0;
-  float fx = 0.f, fy = 0.f, fz = 0.f;
-  LJPairF P = d.ljf[0];
-  const int ntypes = d.ntypes;
-  const size_t cap = d.cap;
-  auto pair = [&](const int4 pj) {
-    const float dx = wrapped_diff(pi.x, pj.x, ux);
-    const float dy = wrapped_diff(pi.y, pj.y, uy);
-    const float dz = wrapped_diff(pi.z, pj.z, uz);
-    const float r2 = dx * dx + dy * dy + dz * dz;
-    if (!SINGLE) P = sP[pi.w * ntypes + pj.w];
-    const float ri2 = fast_rcp(r2);
-    const float ri6 = ri2 * ri2 * ri2;
-    float ff = ri6 * (P.ff1 * ri6 - P.ff2) * ri2;
-    if (CAPPED && r2 <= P.capsq) ff = P.capff * rsqrtf(r2);
+  const int4 pi = ld_pos<LIVE>(&posq[i]);
+  const unsigned long long ux = f2_pack(d.fixUnit[0], d.fixUnit[0]);
+  const unsigned long long uy = f2_pack(d.fixUnit[1], d.fixUnit[1]);
+  const unsigned long long uz = f2_pack(d.fixUnit[2], d.fixUnit[2]);
+  const LJPairF P = d.ljf[0];
+  const unsigned long long ff1s = f2_pack(P.ff1, P.ff1), ff2s = f2_pack(-P.ff2, -P.ff2);
+  const LJPairF* const row = sP + (SINGLE ? 0 : pi.w * d.ntypes);
+  unsigned long long fx = 0ull, fy = 0ull, fz = 0ull;
+  auto pairs = [&](const int4 pa, const int4 pb) {
+    const unsigned long long dx =
+        f2_mul(f2_pack(wrapped_diff(pi.x, pa.x), wrapped_diff(pi.x, pb.x)), ux);
+    const unsigned long long dy =
+        f2_mul(f2_pack(wrapped_diff(pi.y, pa.y), wrapped_diff(pi.y, pb.y)), uy);
+    const unsigned long long dz =
+        f2_mul(f2_pack(wrapped_diff(pi.z, pa.z), wrapped_diff(pi.z, pb.z)), uz);
+    const unsigned long long r2 = f2_fma(dz, dz, f2_fma(dy, dy, f2_mul(dx, dx)));
+    const float ra = f2_lo(r2), rb = f2_hi(r2);
+    unsigned long long c1 = ff1s, c2 = ff2s;
+    LJPairF Pa = P, Pb = P;
+    if (!SINGLE) {
+      Pa = row[pa.w];
+      Pb = row[pb.w];
+      c1 = f2_pack(Pa.ff1, Pb.ff1);
+      c2 = f2_pack(-Pa.ff2, -Pb.ff2);
+    }
+    const unsigned long long ri2 = f2_pack(fast_rcp(ra), fast_rcp(rb));
+    const unsigned long long ri6 = f2_mul(f2_mul(ri2, ri2), ri2);
+    const unsigned long long ff = f2_mul(f2_mul(ri6, f2_fma(c1, ri6, c2)), ri2);
+    float fa = f2_lo(ff), fb = f2_hi(ff);
+    if (CAPPED) {
+      if (ra <= Pa.capsq) fa = Pa.capff * rsqrtf(ra);
+      if (rb <= Pb.capsq) fb = Pb.capff * rsqrtf(rb);
+    }
     // padding entries are the particle itself: r^2 = 0
-    ff = (r2 > 0.f && r2 <= P.rcsq) ? ff : 0.f;
-    fx += dx * ff;
-    fy += dy * ff;
-    fz += dz * ff;
+    fa = (ra > 0.f && ra <= Pa.rcsq) ? fa : 0.f;
+    fb = (rb > 0.f && rb <= Pb.rcsq) ? fb : 0.f;
+    const unsigned long long f = f2_pack(fa, fb);
+    fx = f2_fma(dx, f, fx);
+    fy = f2_fma(dy, f, fy);
+    fz = f2_fma(dz, f, fz);
   };
-  if (TPP == 1) {
-    // The list is padded to a multiple of 8 (with the particle itself), so it is read in
-    // whole blocks of 8: two 16-byte streaming loads per block.  The next block is loaded
-    // before the current block's coordinates are used, so list loads, coordinate gathers
-    // and arithmetic overlap; the sum order is the list order.
-    const int nblk = (cnt + 7) >> 3;
-    const int4* blk = reinterpret_cast<const int4*>(d.nl) + (size_t)i * 2;
-    const size_t bstride = cap * 2;
-    int4 ja = make_int4(i, i, i, i), jb = ja;
-    if (nblk > 0) {
-      ja = ld_list(blk);
-      jb = ld_list(blk + 1);
-    }
-    for (int b = 0; b < nblk; ++b) {
-      const int j[8] = {ja.x, ja.y, ja.z, ja.w, jb.x, jb.y, jb.z, jb.w};
-      int4 pj[8];
+  share.walk(d, i, sub, act ? d.nn[i] : 0, [&](const int (&j)[Share::ENT], auto next) {
+    int4 q[Share::ENT];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) pj[u] = __ldg(&d.posq[j[u]]);
-      blk += bstride;
-      if (b + 1 < nblk) {
-        ja = ld_list(blk);
-        jb = ld_list(blk + 1);
-      }
+    for (int u = 0; u < Share::ENT; ++u) q[u] = ld_pos<LIVE>(&posq[j[u]]);
+    next();
 #pragma unroll
-      for (int u = 0; u < 8; ++u) pair(pj[u]);
-    }
-  } else {
-    // thread sub of particle i takes the blocks sub, sub + TPP, ... (8 entries each, two
-    // 16-byte loads); TPP threads per particle keep TPP list blocks in flight per particle
-    const int nblk = (cnt + 7) >> 3;
-    const int4* blk = reinterpret_cast<const int4*>(d.nl) + ((size_t)sub * cap + i) * 2;
-    const size_t bstride = cap * 2 * TPP;
-    int4 ja = make_int4(i, i, i, i), jb = ja;
-    if (sub < nblk) {
-      ja = ld_list(blk);
-      jb = ld_list(blk + 1);
-    }
-    for (int b = sub; b < nblk; b += TPP) {
-      const int j[8] = {ja.x, ja.y, ja.z, ja.w, jb.x, jb.y, jb.z, jb.w};
-      int4 pj[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) pj[u] = __ldg(&d.posq[j[u]]);
-      blk += bstride;
-      if (b + TPP < nblk) {
-        ja = ld_list(blk);
-        jb = ld_list(blk + 1);
-      }
-#pragma unroll
-      for (int u = 0; u < 8; ++u) pair(pj[u]);
-    }
-  }
-  long long Fx = to_fix(fx, d.err), Fy = to_fix(fy, d.err), Fz = to_fix(fz, d.err);
-  if (FENE && sub == 0 && act) {
+    for (int u = 0; u < Share::ENT; u += 2) pairs(q[u], q[u + 1]);
+  });
+  long long Fx = to_fix(f2_lo(fx) + f2_hi(fx), d.err), Fy = to_fix(f2_lo(fy) + f2_hi(fy), d.err),
+            Fz = to_fix(f2_lo(fz) + f2_hi(fz), d.err);
+  if (FENE && act) {
+    // the particle's bonds, shared out among its lanes
     const int64_t off = a.id[i] - d.idMin;
-    const int b0 = d.bondStart[off], b1 = d.bondStart[off + 1];
+    const int b0 = d.bondStart[off] + sub, b1 = d.bondStart[off + 1];
     float bx = 0.f, by = 0.f, bz = 0.f, bmax = 0.f;
     const float rmaxsq = (float)fp.rmaxsq, K = (float)fp.K, r0 = (float)fp.r0;
-    for (int b = b0; b < b1; ++b) {
+    for (int b = b0; b < b1; b += T) {
       const int64_t po = d.bondPartner[b] - d.idMin;
       const int j = (po >= 0 && po < d.idSpan) ? d.id2idx[po] : -1;
       if (j < 0) {
         atomicOr(d.err, kErrBondMissing);
         continue;
       }
-      const int4 pj = d.posq[j];
-      const float dx = wrapped_diff(pi.x, pj.x, ux);
-      const float dy = wrapped_diff(pi.y, pj.y, uy);
-      const float dz = wrapped_diff(pi.z, pj.z, uz);
+      const int4 pj = ld_pos<LIVE>(&posq[j]);
+      const float dx = wrapped_diff(pi.x, pj.x, d.fixUnit[0]);
+      const float dy = wrapped_diff(pi.y, pj.y, d.fixUnit[1]);
+      const float dz = wrapped_diff(pi.z, pj.z, d.fixUnit[2]);
       const float r2 = dx * dx + dy * dy + dz * dz;
       bmax = fmaxf(bmax, r2);
       if (!(r2 <= (float)fp.rcsq)) continue;
@@ -1134,18 +1128,34 @@ __global__ void __launch_bounds__(256) k_force_mixed(DevView d, FENEParams fp) {
     Fy += to_fix(by, d.err);
     Fz += to_fix(bz, d.err);
   }
-  if (TPP > 1) {
 #pragma unroll
-    for (int o = TPP / 2; o > 0; o >>= 1) {
-      Fx += __shfl_xor_sync(0xffffffffu, Fx, o, TPP);
-      Fy += __shfl_xor_sync(0xffffffffu, Fy, o, TPP);
-      Fz += __shfl_xor_sync(0xffffffffu, Fz, o, TPP);
-    }
+  for (int o = T / 2; o > 0; o >>= 1) {
+    Fx += __shfl_xor_sync(0xffffffffu, Fx, o, T);
+    Fy += __shfl_xor_sync(0xffffffffu, Fy, o, T);
+    Fz += __shfl_xor_sync(0xffffffffu, Fz, o, T);
   }
-  if (sub == 0 && act) {
-    d.ffix[i] = Fx;
-    d.ffix[(size_t)d.cap + i] = Fy;
-    d.ffix[2 * (size_t)d.cap + i] = Fz;
+  F[0] = Fx;
+  F[1] = Fy;
+  F[2] = Fz;
+}
+
+template <int T, bool SINGLE, bool CAPPED, bool FENE>
+__global__ void __launch_bounds__(256, kMixMB) k_force_mixed(DevView d, FENEParams fp) {
+  __shared__ LJPairF sP[kMaxTypes * kMaxTypes];
+  if (!SINGLE) {
+    for (int t = threadIdx.x; t < d.ntypes * d.ntypes; t += blockDim.x) sP[t] = d.ljf[t];
+    __syncthreads();
+  }
+  const int gt = blockIdx.x * blockDim.x + threadIdx.x;
+  if (T == 1 && gt >= d.n) return;
+  const bool act = gt / T < d.n;
+  const int i = act ? gt / T : 0;
+  long long F[3];
+  particle_force_mixed<T, SINGLE, CAPPED, FENE, false>(d, fp, sP, d.posq, i, gt % T, act,
+                                                       ListShare<T>(), F);
+  if (gt % T == 0 && act) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) d.ffix[c * (size_t)d.cap + i] = F[c];
   }
 }
 
@@ -1157,82 +1167,107 @@ __device__ __forceinline__ double min_image(double dx, double L, double halfL) {
   return dx;
 }
 
+// 1 / x by Newton's iteration on the hardware's approximate reciprocal, the quadratic and
+// cubic terms of the error e = 1 - x r0 taken together: r0 (1 + e + e^2) leaves e^3, below
+// the rounding of the result.  For a pair's r^2 only: no special values.
+__device__ __forceinline__ double pair_rcp(double x) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double e = fma(-x, r, 1.0);
+  return fma(r, fma(e, e, e), r);
+}
+
+// 1 / sqrt(x) in the same way: y0 from the hardware, e = 1 - x y0^2, y0 (1 + e/2 + 3 e^2 / 8).
+__device__ __forceinline__ double pair_rsqrt(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x * y, y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
 // Plain FP64 form of the same kernel (reference arithmetic of LennardJones.hpp:137-143
-// and FENE.hpp:97-112 on minimum-image distances).
-template <int TPP, bool SINGLE, bool CAPPED, bool FENE>
-__global__ void __launch_bounds__(256) k_force_fp64(DevView d, FENEParams fp) {
+// and FENE.hpp:97-112 on minimum-image distances).  A warp whose particles all lie farther
+// than wrapMargin from every face of the box has no partner across one: its differences are
+// their own minimum images, bit for bit, and the 12 FP64 instructions of the comparisons
+// and shifts (of 30 a pair) are skipped.  The reciprocal is Newton steps on the hardware's
+// approximation instead of a division.  Bound by the FP64 pipe and the gathers: 402 us before
+// and 192 now at 1,009,091 particles (one type), 19.8 and 13 at 32,768.  Registers: four
+// blocks an SM with one type (203 us with three), three where the pair's constants are loaded
+// per entry.
+template <int T, bool SINGLE, bool CAPPED, bool FENE, bool LIVE, class Share>
+__device__ __forceinline__ void particle_force_fp64(const DevView& d, const FENEParams& fp,
+                                                    const double* X, int i, int sub, bool act,
+                                                    const Share& share, double (&F)[3]) {
   const ParticleArrays a = d.pa[0];
-  const int gt = blockIdx.x * blockDim.x + threadIdx.x;
-  const int i0 = gt / TPP;
-  const int sub = gt % TPP;
-  if (TPP == 1 && i0 >= d.n) return;
-  const bool act = i0 < d.n;
-  const int i = act ? i0 : 0;
-  const double* X = a.x;
-  const double* Y = a.x + d.cap;
-  const double* Z = a.x + 2 * (size_t)d.cap;
-  const double xi = X[i], yi = Y[i], zi = Z[i];
-  const int ti = a.type[i];
-  const int cnt = act ? d.nn[i] : 0;
+  const double* Y = X + d.cap;
+  const double* Z = X + 2 * (size_t)d.cap;
+  const double xi = ld_pos<LIVE>(&X[i]), yi = ld_pos<LIVE>(&Y[i]), zi = ld_pos<LIVE>(&Z[i]);
+  const LJPair* const row = d.lj + (SINGLE ? 0 : a.type[i] * d.ntypes);
+  const double sc1 = d.lj[0].ff1, sc2 = d.lj[0].ff2, srcsq = d.lj[0].rcsq;
   double fx = 0, fy = 0, fz = 0;
-  const int ntypes = d.ntypes;
-  const size_t cap = d.cap;
-  auto pair = [&](int j, double xj, double yj, double zj) {
-    const double dx = min_image(xi - xj, d.L[0], d.halfL[0]);
-    const double dy = min_image(yi - yj, d.L[1], d.halfL[1]);
-    const double dz = min_image(zi - zj, d.L[2], d.halfL[2]);
+  auto pair = [&](double dx, double dy, double dz, int tj) {
     const double r2 = dx * dx + dy * dy + dz * dz;
-    const LJPair& P = SINGLE ? d.lj[0] : d.lj[ti * ntypes + __ldg(&a.type[j])];
-    if (!P.set || !(r2 > 0.0) || r2 > P.rcsq) return;  // padding: the particle itself
-    double ff;
-    if (CAPPED && P.caprad > 0 && !(r2 > P.caprad * P.caprad)) {
-      ff = P.capff / sqrt(r2);
-    } else {
-      const double ri2 = 1.0 / r2;
-      const double ri6 = ri2 * ri2 * ri2;
-      ff = ri6 * (P.ff1 * ri6 - P.ff2) * ri2;
+    const LJPair& P = row[SINGLE ? 0 : tj];
+    const double c1 = SINGLE ? sc1 : P.ff1, c2 = SINGLE ? sc2 : P.ff2;
+    // padding entries are the particle itself: r^2 = 0
+    bool in = r2 > 0.0 && !(r2 > (SINGLE ? srcsq : P.rcsq));
+    if (!SINGLE) in = in && P.set;
+    const double ri2 = pair_rcp(r2);
+    const double ri6 = ri2 * ri2 * ri2;
+    double ff = ri6 * (c1 * ri6 - c2) * ri2;
+    if (CAPPED && P.caprad > 0 && !(r2 > P.caprad * P.caprad)) ff = P.capff / sqrt(r2);
+    if (in) {
+      fx += dx * ff;
+      fy += dy * ff;
+      fz += dz * ff;
     }
-    fx += dx * ff;
-    fy += dy * ff;
-    fz += dz * ff;
   };
-  {
-    // thread sub of particle i takes the blocks sub, sub + TPP, ... (8 entries each, read
-    // as two 16-byte loads)
-    const int nblk = (cnt + 7) >> 3;
-    const int4* blk = reinterpret_cast<const int4*>(d.nl) + ((size_t)sub * cap + i) * 2;
-    const size_t bstride = cap * 2 * TPP;
-    for (int b = sub; b < nblk; b += TPP, blk += bstride) {
+  auto loop = [&](auto wrap) {
+    share.walk(d, i, sub, act ? d.nn[i] : 0, [&](const int (&j)[Share::ENT], auto next) {
+      double xj[Share::ENT], yj[Share::ENT], zj[Share::ENT];
+      int tj[Share::ENT];
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int4 jj = __ldcs(blk + h);
-        const int j[4] = {jj.x, jj.y, jj.z, jj.w};
-        double xj[4], yj[4], zj[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          xj[u] = __ldg(&X[j[u]]);
-          yj[u] = __ldg(&Y[j[u]]);
-          zj[u] = __ldg(&Z[j[u]]);
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) pair(j[u], xj[u], yj[u], zj[u]);
+      for (int u = 0; u < Share::ENT; ++u) {
+        xj[u] = ld_pos<LIVE>(&X[j[u]]);
+        yj[u] = ld_pos<LIVE>(&Y[j[u]]);
+        zj[u] = ld_pos<LIVE>(&Z[j[u]]);
+        tj[u] = SINGLE ? 0 : __ldg(&a.type[j[u]]);
       }
-    }
-  }
-  if (FENE && sub == 0 && act) {
+      next();
+#pragma unroll
+      for (int u = 0; u < Share::ENT; ++u) {
+        double dx = xi - xj[u], dy = yi - yj[u], dz = zi - zj[u];
+        if (decltype(wrap)::value) {
+          dx = min_image(dx, d.L[0], d.halfL[0]);
+          dy = min_image(dy, d.L[1], d.halfL[1]);
+          dz = min_image(dz, d.L[2], d.halfL[2]);
+        }
+        pair(dx, dy, dz, tj[u]);
+      }
+    });
+  };
+  const double m = d.wrapMargin;
+  const bool inner = xi > m && xi < d.L[0] - m && yi > m && yi < d.L[1] - m && zi > m &&
+                     zi < d.L[2] - m;
+  if (__all_sync(0xffffffffu, inner || !act))
+    loop(std::false_type{});
+  else
+    loop(std::true_type{});
+  if (FENE && act) {
+    // the particle's bonds, shared out among its lanes
     const int64_t off = a.id[i] - d.idMin;
-    const int b0 = d.bondStart[off], b1 = d.bondStart[off + 1];
+    const int b0 = d.bondStart[off] + sub, b1 = d.bondStart[off + 1];
     double bmax = 0.0;
-    for (int b = b0; b < b1; ++b) {
+    for (int b = b0; b < b1; b += T) {
       const int64_t po = d.bondPartner[b] - d.idMin;
       const int j = (po >= 0 && po < d.idSpan) ? d.id2idx[po] : -1;
       if (j < 0) {
         atomicOr(d.err, kErrBondMissing);
         continue;
       }
-      const double dx = min_image(xi - X[j], d.L[0], d.halfL[0]);
-      const double dy = min_image(yi - Y[j], d.L[1], d.halfL[1]);
-      const double dz = min_image(zi - Z[j], d.L[2], d.halfL[2]);
+      const double dx = min_image(xi - ld_pos<LIVE>(&X[j]), d.L[0], d.halfL[0]);
+      const double dy = min_image(yi - ld_pos<LIVE>(&Y[j]), d.L[1], d.halfL[1]);
+      const double dz = min_image(zi - ld_pos<LIVE>(&Z[j]), d.L[2], d.halfL[2]);
       const double r2 = dx * dx + dy * dy + dz * dz;
       bmax = fmax(bmax, r2);
       if (r2 > fp.rcsq) continue;
@@ -1249,18 +1284,28 @@ __global__ void __launch_bounds__(256) k_force_fp64(DevView d, FENEParams fp) {
     }
     if (b1 > b0) note_bond_sq(d.ctr, bmax);
   }
-  if (TPP > 1) {
 #pragma unroll
-    for (int o = TPP / 2; o > 0; o >>= 1) {
-      fx += __shfl_xor_sync(0xffffffffu, fx, o, TPP);
-      fy += __shfl_xor_sync(0xffffffffu, fy, o, TPP);
-      fz += __shfl_xor_sync(0xffffffffu, fz, o, TPP);
-    }
+  for (int o = T / 2; o > 0; o >>= 1) {
+    fx += __shfl_xor_sync(0xffffffffu, fx, o, T);
+    fy += __shfl_xor_sync(0xffffffffu, fy, o, T);
+    fz += __shfl_xor_sync(0xffffffffu, fz, o, T);
   }
-  if (sub == 0 && act) {
-    d.f64[i] = fx;
-    d.f64[(size_t)d.cap + i] = fy;
-    d.f64[2 * (size_t)d.cap + i] = fz;
+  F[0] = fx;
+  F[1] = fy;
+  F[2] = fz;
+}
+
+template <int T, bool SINGLE, bool CAPPED, bool FENE>
+__global__ void __launch_bounds__(256, SINGLE ? 4 : 3) k_force_fp64(DevView d, FENEParams fp) {
+  const int gt = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool act = gt / T < d.n;  // every lane stays for the vote and the shuffles
+  const int i = act ? gt / T : 0;
+  double F[3];
+  particle_force_fp64<T, SINGLE, CAPPED, FENE, false>(d, fp, d.pa[0].x, i, gt % T, act,
+                                                      ListShare<T>(), F);
+  if (gt % T == 0 && act) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) d.f64[c * (size_t)d.cap + i] = F[c];
   }
 }
 
