@@ -196,6 +196,12 @@ struct DevView {
   DevCounters* ctr;       // step-loop state
 };
 
+// Shared state of the one-launch step loop of a small system (k_steps).
+struct StepSync {
+  alignas(128) unsigned long long count;  // grid barrier: blocks arrived so far
+  alignas(128) unsigned long long maxSq[3];  // largest |dx|^2 of a step, three slots in turn
+};
+
 struct RebuildScratch {
   int32_t* cellOf;    // cap: cell of particle (unsorted order)
   int32_t* slot;      // cap: arrival slot inside its cell
@@ -230,6 +236,15 @@ void launch_wait_selftest(unsigned* err, long long spins, unsigned long long* ou
                           cudaStream_t st);
 void launch_integrate(const DevView& d, const IntegrateArgs& a, cudaStream_t st);
 // maxDist += sqrt(max |dx|^2); flag = maxDist > skinHalf
+// Every step up to the next re-sort or the end of the run as one cooperative launch; sets the
+// conditionals of the captured loop.  sync: zeroed before the run; posqAlt: second buffer of
+// packed coordinates.
+cudaError_t launch_steps(const DevView& d, bool mixed, const FENEParams& fene,
+                         const IntegrateArgs& a, double skinHalf, StepSync* sync, int4* posqAlt,
+                         cudaGraphConditionalHandle hIf, cudaGraphConditionalHandle hWhile,
+                         int tpp, int nsm, cudaStream_t st);
+constexpr int kStepParticles = 65536;  // 16-bit list entries in shared memory
+int step_threads(bool mixed);          // lanes of the one block an SM runs
 void launch_decide(const DevView& d, double skinHalf, cudaStream_t st);
 // graph form: also advances ctr->step / ctr->remaining and sets the conditionals
 void launch_decide_graph(const DevView& d, double skinHalf, cudaGraphConditionalHandle hIf,

@@ -1317,9 +1317,70 @@ __device__ __forceinline__ double warp_max(double v) {
   return v;
 }
 
-// aftCalcF (LangevinThermostat::frictionThermo, CapForce) on the pair force, then
-// integrate2 of this step and integrate1 of the next (VelocityVerlet.cpp:236-305),
-// with the reference's operation order and no FMA contraction.
+// aftCalcF (LangevinThermostat::frictionThermo, CapForce) on the pair force F of one
+// particle, then integrate2 of this step and integrate1 of the next
+// (VelocityVerlet.cpp:236-305), with the reference's operation order and no FMA contraction.
+// F becomes the total force; returns |dx|^2 of integrate1 (0 without it).
+__device__ __forceinline__ double advance(const IntegrateArgs& a, int64_t id, bool thermo, double m,
+                                          double (&F)[3], double (&v)[3], double (&x)[3]) {
+  if (thermo) {
+    const double massf = sqrt(m);
+    double u[3];
+    langevin_uniforms(a.seed, id, a.step, a.phase, u);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const double t1 = __dmul_rn(__dmul_rn(a.pref1, v[k]), m);
+      const double t2 = __dmul_rn(__dmul_rn(a.pref2, u[k] - 0.5), massf);
+      F[k] = __dadd_rn(F[k], __dadd_rn(t1, t2));
+    }
+  }
+  if (a.capMode == 1) {
+    const double capfsq = __dmul_rn(a.cap[0], a.cap[0]);
+    const double fsq =
+        __dadd_rn(__dadd_rn(__dmul_rn(F[0], F[0]), __dmul_rn(F[1], F[1])), __dmul_rn(F[2], F[2]));
+    if (fsq > capfsq) {
+      const double scaling = sqrt(capfsq / fsq);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) F[k] = __dmul_rn(F[k], scaling);
+    }
+  } else if (a.capMode == 2) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      if (F[k] > 0 && F[k] > a.cap[k])
+        F[k] = a.cap[k];
+      else if (F[k] < 0 && F[k] < -a.cap[k])
+        F[k] = -a.cap[k];
+    }
+  }
+  const double dtfm = __ddiv_rn(__dmul_rn(0.5, a.dt), m);
+  if (a.do_i2) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) v[k] = __dadd_rn(v[k], __dmul_rn(dtfm, F[k]));
+  }
+  if (!a.do_i1) return 0.0;
+  double dp[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    v[k] = __dadd_rn(v[k], __dmul_rn(dtfm, F[k]));
+    dp[k] = __dmul_rn(v[k], a.dt);
+    x[k] = __dadd_rn(x[k], dp[k]);
+  }
+  return __dadd_rn(__dadd_rn(__dmul_rn(dp[0], dp[0]), __dmul_rn(dp[1], dp[1])),
+                   __dmul_rn(dp[2], dp[2]));
+}
+
+// The block's largest sq into *maxSq (bits of a non-negative double order like integers).
+__device__ __forceinline__ void block_max_sq(double sq, double* smax, unsigned long long* maxSq) {
+  sq = warp_max(sq);
+  if ((threadIdx.x & 31) == 0) smax[threadIdx.x >> 5] = sq;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    double v = threadIdx.x < blockDim.x / 32 ? smax[threadIdx.x] : 0.0;
+    v = warp_max(v);
+    if (threadIdx.x == 0 && v > 0.0) atomicMax(maxSq, (unsigned long long)__double_as_longlong(v));
+  }
+}
+
 template <bool MIXED>
 __global__ void __launch_bounds__(256) k_integrate(DevView d, IntegrateArgs a) {
   const ParticleArrays P = d.pa[0];
@@ -1338,64 +1399,22 @@ __global__ void __launch_bounds__(256) k_integrate(DevView d, IntegrateArgs a) {
   if (i < d.n && !(d.halo && d.halo[P.id[i] - d.idMin])) {  // halo copies stay put
     const size_t cap = d.cap;
     const double m = P.mass[i];
-    double F[3], v[3], x[3];
+    double F[3], v[3], x[3] = {0, 0, 0};
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
       F[k] = MIXED ? (double)d.ffix[k * cap + i] * kInvFix : d.f64[k * cap + i];
       v[k] = P.v[k * cap + i];
+      if (a.do_i1) x[k] = P.x[k * cap + i];
     }
-    if (a.langevin) {
-      const int64_t id = P.id[i];
-      if (!(d.langExcl && d.langExcl[id - d.idMin])) {
-        const double massf = sqrt(m);
-        double u[3];
-        langevin_uniforms(a.seed, id, a.step, a.phase, u);
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          const double t1 = __dmul_rn(__dmul_rn(a.pref1, v[k]), m);
-          const double t2 = __dmul_rn(__dmul_rn(a.pref2, u[k] - 0.5), massf);
-          F[k] = __dadd_rn(F[k], __dadd_rn(t1, t2));
-        }
-      }
-    }
-    if (a.capMode == 1) {
-      const double capfsq = __dmul_rn(a.cap[0], a.cap[0]);
-      const double fsq =
-          __dadd_rn(__dadd_rn(__dmul_rn(F[0], F[0]), __dmul_rn(F[1], F[1])), __dmul_rn(F[2], F[2]));
-      if (fsq > capfsq) {
-        const double scaling = sqrt(capfsq / fsq);
-#pragma unroll
-        for (int k = 0; k < 3; ++k) F[k] = __dmul_rn(F[k], scaling);
-      }
-    } else if (a.capMode == 2) {
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        if (F[k] > 0 && F[k] > a.cap[k])
-          F[k] = a.cap[k];
-        else if (F[k] < 0 && F[k] < -a.cap[k])
-          F[k] = -a.cap[k];
-      }
-    }
+    const int64_t id = a.langevin ? P.id[i] : 0;
+    sq = advance(a, id, a.langevin && !(d.langExcl && d.langExcl[id - d.idMin]), m, F, v, x);
     if (a.storeFtot) {
 #pragma unroll
       for (int k = 0; k < 3; ++k) d.ftot[k * cap + i] = F[k];
     }
-    const double dtfm = __ddiv_rn(__dmul_rn(0.5, a.dt), m);
-    if (a.do_i2) {
-#pragma unroll
-      for (int k = 0; k < 3; ++k) v[k] = __dadd_rn(v[k], __dmul_rn(dtfm, F[k]));
-    }
     if (a.do_i1) {
-      double dp[3];
 #pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        v[k] = __dadd_rn(v[k], __dmul_rn(dtfm, F[k]));
-        dp[k] = __dmul_rn(v[k], a.dt);
-        x[k] = __dadd_rn(P.x[k * cap + i], dp[k]);
-        P.x[k * cap + i] = x[k];
-      }
-      sq = __dadd_rn(__dadd_rn(__dmul_rn(dp[0], dp[0]), __dmul_rn(dp[1], dp[1])),
-                     __dmul_rn(dp[2], dp[2]));
+      for (int k = 0; k < 3; ++k) P.x[k * cap + i] = x[k];
       d.posq[i] = fixed_coords(d, x[0], x[1], x[2], P.type[i]);
     }
     if (a.do_i1 || a.do_i2) {
@@ -1403,17 +1422,7 @@ __global__ void __launch_bounds__(256) k_integrate(DevView d, IntegrateArgs a) {
       for (int k = 0; k < 3; ++k) P.v[k * cap + i] = v[k];
     }
   }
-  if (a.do_i1) {
-    sq = warp_max(sq);
-    if ((threadIdx.x & 31) == 0) smax[threadIdx.x >> 5] = sq;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-      double v = threadIdx.x < blockDim.x / 32 ? smax[threadIdx.x] : 0.0;
-      v = warp_max(v);
-      if (threadIdx.x == 0 && v > 0.0)
-        atomicMax(&d.ctr->maxSq, (unsigned long long)__double_as_longlong(v));
-    }
-  }
+  if (a.do_i1) block_max_sq(sq, smax, &d.ctr->maxSq);
 }
 
 __device__ __forceinline__ int decide_core(DevCounters* c, double skinHalf) {
@@ -1439,6 +1448,238 @@ __global__ void k_decide_graph(DevCounters* c, double skinHalf, cudaGraphConditi
   const int f = decide_core(c, skinHalf);
   cudaGraphSetConditional(hIf, f ? 1u : 0u);
   cudaGraphSetConditional(hWhile, rem > 0 ? 1u : 0u);
+}
+
+constexpr int kBarrierTries = 1 << 21;  // about a second
+
+// ---- steps of a small system ------------------------------------------------------------
+// All steps up to the next re-sort or the end of the run in one cooperative launch.  A small
+// system's step is bound by launches and by the tail of each kernel, not by its work: the
+// force, integrate and decide kernels of 32,768 particles take 15 us a step, most of it
+// latency.  Here the lanes that sum a particle's force also advance it, and one barrier over
+// the grid ends the step; positions alternate between two buffers, so a step reads the old
+// ones while it writes the new ones.  The largest displacement goes through three slots in
+// turn (one being raised, one read, one cleared).  Every block takes the same decision from
+// the same numbers; block 0 writes it down.
+// The result is that of the separate kernels, bit for bit: the same arithmetic with the same
+// lanes a particle.  A step without re-sorts takes 6.3 us at 1,728 particles and 9.6 (mixed) or
+// 12.0 (FP64) at 32,768.  With re-sorts, separate kernels against this one: mixed 18.5 / 13.3 us
+// a step at 8,000 particles, 24.5 / 18.9 at 32,768, 32.0 / 26.2 at 64,000; FP64 21.2 / 14.1 at
+// 8,000 and 33.8 / 26.0 at 46,656.
+// A step's chain of L2 round trips is its cost, so the barrier is one counter that only grows
+// (the blocks arrive on it and poll it), and the thread that polled also fetches *word, the
+// value every thread wants next.  passed: barriers passed so far times the grid's blocks.
+__device__ __forceinline__ bool grid_barrier(StepSync* s, unsigned long long& passed,
+                                             const unsigned long long* word, double& value,
+                                             unsigned* err) {
+  __shared__ bool s_ok;
+  __shared__ unsigned long long s_word;
+  passed += gridDim.x;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    // the barriers of the block order its threads' accesses before the release here and
+    // behind the acquire below
+    unsigned long long now;
+    asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(&s->count) : "memory");
+    int tries = 0;
+    do {
+      asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(now) : "l"(&s->count) : "memory");
+    } while (now < passed && ++tries < kBarrierTries);
+    s_ok = now >= passed;
+    if (!s_ok) atomicOr(err, kErrTimeout);
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(s_word) : "l"(word) : "memory");
+  }
+  __syncthreads();
+  value = __longlong_as_double((long long)s_word);
+  return s_ok;
+}
+
+// Threads of the one block an SM runs: what the registers of the force loop allow (64 in
+// FP32, 96 in FP64).
+template <bool MIXED>
+constexpr int kStepThreads = MIXED ? 1024 : 640;
+
+// A lane's share of a list kept in shared memory for the whole launch, as 16-bit indices two a
+// word (the step kernel's systems hold at most 65,536 particles): blocks of 8 entries as in
+// ListShare, a particle's words contiguous with a stride of 52, so the lanes of a warp fall on
+// different banks.  The entries come in the order of ListShare, B of them a step: a barrier
+// over the grid drops the SM's L1, so a step's chain is list, coordinates, sums, and both fewer
+// round trips and more gathers in flight shorten it.  Blocks beyond the stage are read from
+// the list itself.
+constexpr int kStepWords = 52, kStepBlocks = kStepWords / 4;
+
+template <int T, int B>
+struct StepShare {
+  static constexpr int E = T == 1 ? 8 : (T == 2 ? 4 : 2);  // entries of a block a lane takes
+  static constexpr int ENT = B;
+  static constexpr int U = B / E;                          // blocks of one step
+  static constexpr int kStride = T == 8 ? 2 : 1;
+  const uint32_t* words;  // the particle's words
+
+  template <class F>
+  __device__ __forceinline__ void walk(const DevView& d, int i, int sub, int cnt, F&& f) const {
+    const int nblk = (cnt + 7) >> 3, first = T == 8 ? sub >> 2 : 0;
+    const int lane = T >= 4 ? (sub & 3) * 2 : sub * E;  // first entry inside a block
+    for (int b = first; b < nblk; b += U * kStride) {
+      int j[ENT];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int k = b + u * kStride;
+#pragma unroll
+        for (int e = 0; e < E; e += 2) {
+          int j0 = i, j1 = i;
+          if (k < nblk) {
+            if (k < kStepBlocks) {
+              const uint32_t w = words[4 * k + (lane + e) / 2];
+              j0 = (int)(w & 0xffffu);
+              j1 = (int)(w >> 16);
+            } else {
+              const int2 v = ld_list2(reinterpret_cast<const int2*>(
+                  d.nl + nl_index(8 * k, i, d.cap) + lane + e));
+              j0 = v.x;
+              j1 = v.y;
+            }
+          }
+          j[u * E + e] = j0;
+          j[u * E + e + 1] = j1;
+        }
+      }
+      f(j, [] {});
+    }
+  }
+};
+
+template <bool MIXED, int T, bool SINGLE, bool CAPPED, bool FENE>
+__global__ void __launch_bounds__(kStepThreads<MIXED>, 1)
+    k_steps(DevView d, FENEParams fp, IntegrateArgs a, double skinHalf, StepSync* sync,
+            int4* posqAlt, cudaGraphConditionalHandle hIf, cudaGraphConditionalHandle hWhile) {
+  const ParticleArrays P = d.pa[0];
+  double* const xAlt = d.pa[1].x;  // the re-sort's target is free between re-sorts
+  __shared__ LJPairF sP[kMaxTypes * kMaxTypes];
+  __shared__ double smax[kStepThreads<MIXED> / 32];
+  if (MIXED && !SINGLE)
+    for (int t = threadIdx.x; t < d.ntypes * d.ntypes; t += blockDim.x) sP[t] = d.ljf[t];
+  DevCounters* const c = d.ctr;
+  long long step = c->step, rem = c->remaining;
+  double maxDist = c->maxDist, msq = __longlong_as_double((long long)c->maxSq);
+  bool resume = c->flag != 0;  // the re-sort of this step is done: its force is next
+  // between launches the counter is a multiple of the grid's blocks
+  unsigned long long passed = *(volatile unsigned long long*)&sync->count;
+  passed -= passed % gridDim.x;
+  a.pref1 = c->pref1;
+  a.pref2 = c->pref2;
+  const int gt = blockIdx.x * blockDim.x + threadIdx.x, sub = gt % T;
+  const size_t cap = d.cap;
+  // one particle a group of T lanes (the grid covers them), its list into shared memory
+  const bool act = gt / T < d.n;
+  const int i = act ? gt / T : 0;
+  extern __shared__ uint32_t s_list[];
+  const int perBlock = blockDim.x / T, p0 = blockIdx.x * perBlock;
+  for (int q = threadIdx.x; q < perBlock * kStepWords; q += blockDim.x) {
+    const int p = p0 + q / kStepWords, w = q % kStepWords;
+    if (p >= d.n || 2 * w >= ((d.nn[p] + 7) & ~7)) continue;
+    const int2 v =
+        *reinterpret_cast<const int2*>(d.nl + nl_index(8 * (w >> 2), p, cap) + 2 * (w & 3));
+    s_list[q] = (uint32_t)v.x | (uint32_t)v.y << 16;
+  }
+  const bool thermo = a.langevin && !(d.langExcl && d.langExcl[P.id[i] - d.idMin]);
+  const StepShare<T, MIXED ? 8 : (T == 1 ? 8 : 4)> share{s_list + threadIdx.x / T * kStepWords};
+  bool resort = false, ok = true;
+  int k = 0, slot = 0;  // steps done: the current positions are in the first buffer when even
+  __syncthreads();
+  while (true) {
+    const int4* const posq = k & 1 ? posqAlt : d.posq;
+    int4* const posqNew = k & 1 ? d.posq : posqAlt;
+    const double* const X = k & 1 ? xAlt : P.x;
+    double* const xNew = k & 1 ? P.x : xAlt;
+    if (sub == 0) {  // under way while the step is decided; read behind the pair loop
+      if (MIXED) prefetch_l1(&posq[i]);
+      prefetch_l1(&P.mass[i]);
+      prefetch_l1(&P.id[i]);
+      prefetch_l1(&P.type[i]);
+#pragma unroll
+      for (int e = 0; e < 3; ++e) {
+        prefetch_l1(&P.v[e * cap + i]);
+        prefetch_l1(&(MIXED ? P.x : X)[e * cap + i]);
+      }
+    }
+    if (!resume) {
+      ++step;
+      --rem;
+      const double md = __dadd_rn(maxDist, sqrt(msq));
+      resort = md > skinHalf;
+      maxDist = resort ? 0.0 : md;
+      if (resort) break;
+    }
+    resume = false;
+    a.step = step;
+    a.do_i1 = rem > 0 ? 1 : 0;
+    double sq = 0.0;
+    double F[3];
+    if (MIXED) {
+      long long G[3];
+      particle_force_mixed<T, SINGLE, CAPPED, FENE, true>(d, fp, sP, posq, i, sub, act, share, G);
+#pragma unroll
+      for (int e = 0; e < 3; ++e) F[e] = (double)G[e] * kInvFix;
+    } else {
+      particle_force_fp64<T, SINGLE, CAPPED, FENE, true>(d, fp, X, i, sub, act, share, F);
+    }
+    if (sub == 0 && act) {
+      double v[3], x[3];
+#pragma unroll
+      for (int e = 0; e < 3; ++e) {
+        v[e] = P.v[e * cap + i];
+        x[e] = ld_pos<true>((MIXED ? P.x : X) + e * cap + i);
+      }
+      sq = advance(a, P.id[i], thermo, P.mass[i], F, v, x);
+#pragma unroll
+      for (int e = 0; e < 3; ++e) {
+        P.v[e * cap + i] = v[e];
+        if (a.do_i1) (MIXED ? P.x : xNew)[e * cap + i] = x[e];
+        if (rem == 0) d.ftot[e * cap + i] = F[e];
+      }
+      if (MIXED && a.do_i1) posqNew[i] = fixed_coords(d, x[0], x[1], x[2], P.type[i]);
+    }
+    if (a.do_i1) {
+      block_max_sq(sq, smax, &sync->maxSq[slot]);
+      if (gt == 0) sync->maxSq[slot == 2 ? 0 : slot + 1] = 0ull;
+    }
+    ok = grid_barrier(sync, passed, &sync->maxSq[slot], msq, d.err);
+    if (!ok || rem == 0) break;
+    ++k;
+    slot = slot == 2 ? 0 : slot + 1;
+  }
+  // behind this barrier nobody reads the counters or the slots any more
+  if (resort) ok = grid_barrier(sync, passed, &sync->maxSq[slot], msq, d.err);
+  const bool odd = k & 1;
+  // the run's end: current positions into the first buffer (packed ones are made anew by a
+  // re-sort)
+  if (MIXED ? odd && !resort : odd || !resort) {
+    if (act && sub == 0) {
+      if (MIXED) {
+        d.posq[i] = ld_pos<true>(&posqAlt[i]);
+      } else {
+        double x[3];
+#pragma unroll
+        for (int e = 0; e < 3; ++e) {
+          x[e] = ld_pos<true>((odd ? xAlt : P.x) + e * cap + i);
+          if (odd) P.x[e * cap + i] = x[e];
+        }
+        d.posq[i] = fixed_coords(d, x[0], x[1], x[2], P.type[i]);
+      }
+    }
+  }
+  if (gt == 0) {
+    c->step = step;
+    c->remaining = rem;
+    c->maxDist = maxDist;
+    c->maxSq = 0ull;
+    c->flag = resort ? 1 : 0;
+    c->resorts += resort ? 1 : 0;
+    sync->maxSq[0] = sync->maxSq[1] = sync->maxSq[2] = 0ull;
+    cudaGraphSetConditional(hIf, ok && resort ? 1u : 0u);
+    cudaGraphSetConditional(hWhile, ok && (resort || rem > 0) ? 1u : 0u);
+  }
 }
 
 // ---- observables -------------------------------------------------------------------
@@ -2314,6 +2555,66 @@ void launch_decide(const DevView& d, double skinHalf, cudaStream_t st) {
 void launch_decide_graph(const DevView& d, double skinHalf, cudaGraphConditionalHandle hIf,
                          cudaGraphConditionalHandle hWhile, cudaStream_t st) {
   k_decide_graph<<<1, 1, 0, st>>>(d.ctr, skinHalf, hIf, hWhile);
+}
+
+namespace {
+template <bool MIXED, int T>
+cudaError_t steps_dispatch(const DevView& d, const FENEParams& fp, const IntegrateArgs& a,
+                           double skinHalf, StepSync* sync, int4* posqAlt,
+                           cudaGraphConditionalHandle hIf, cudaGraphConditionalHandle hWhile,
+                           int nsm, cudaStream_t st) {
+  using Kernel = void (*)(DevView, FENEParams, IntegrateArgs, double, StepSync*, int4*,
+                          cudaGraphConditionalHandle, cudaGraphConditionalHandle);
+  const bool single = d.ljSingle != 0, capped = d.ljCapped != 0, fene = fp.on != 0;
+  Kernel f = nullptr;
+#define ESPP_STEPS_CASE(S, C, F) \
+  if (single == S && capped == C && fene == F) f = k_steps<MIXED, T, S, C, F>;
+  ESPP_STEPS_CASE(true, false, false)
+  ESPP_STEPS_CASE(true, false, true)
+  ESPP_STEPS_CASE(true, true, false)
+  ESPP_STEPS_CASE(true, true, true)
+  ESPP_STEPS_CASE(false, false, false)
+  ESPP_STEPS_CASE(false, false, true)
+  ESPP_STEPS_CASE(false, true, false)
+  ESPP_STEPS_CASE(false, true, true)
+#undef ESPP_STEPS_CASE
+  // one block an SM, as large as the particles need to fill them all
+  const long long lanes = (long long)d.n * T;
+  int block = (int)((lanes + nsm - 1) / nsm + 31) / 32 * 32;
+  if (block < 64) block = 64;
+  if (block > kStepThreads<MIXED>) return cudaErrorCooperativeLaunchTooLarge;
+  const size_t smem = sizeof(uint32_t) * kStepWords * (block / T);
+  cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  int perSm = 0;
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, f, block, smem);
+  if (e != cudaSuccess) return e;
+  const int grid = blocks_for(lanes, block);
+  if ((long long)perSm * nsm < grid) return cudaErrorCooperativeLaunchTooLarge;
+  DevView dv = d;
+  FENEParams fv = fp;
+  IntegrateArgs av = a;
+  void* args[] = {&dv, &fv, &av, &skinHalf, &sync, &posqAlt, &hIf, &hWhile};
+  return cudaLaunchCooperativeKernel((const void*)f, dim3(grid), dim3(block), args, smem, st);
+}
+}  // namespace
+
+int step_threads(bool mixed) { return mixed ? kStepThreads<true> : kStepThreads<false>; }
+
+cudaError_t launch_steps(const DevView& d, bool mixed, const FENEParams& fp,
+                         const IntegrateArgs& a, double skinHalf, StepSync* sync, int4* posqAlt,
+                         cudaGraphConditionalHandle hIf, cudaGraphConditionalHandle hWhile,
+                         int tpp, int nsm, cudaStream_t st) {
+#define ESPP_STEPS(T)                                                                        \
+  return mixed ? steps_dispatch<true, T>(d, fp, a, skinHalf, sync, posqAlt, hIf, hWhile, nsm, st) \
+               : steps_dispatch<false, T>(d, fp, a, skinHalf, sync, posqAlt, hIf, hWhile, nsm, st)
+  switch (tpp) {
+    case 1: ESPP_STEPS(1);
+    case 2: ESPP_STEPS(2);
+    case 4: ESPP_STEPS(4);
+    default: ESPP_STEPS(8);
+  }
+#undef ESPP_STEPS
 }
 
 void launch_lj_observables(const DevView& d, double* partials, int nblocks, double* out,

@@ -1,6 +1,8 @@
-"""The size-dependent routes of a re-sort: which list build and which sort kernel runs depends
-on sizes and density.  Each route at the sizes where it can go wrong (partial warps and tiles,
-runs that change row of cells, lists beyond a stage, crowded cells) against the CPU oracle."""
+"""The size-dependent routes of the step: which list build, re-sort, step loop and
+observable kernel runs depends on sizes, types and density.  Each route at the sizes where it
+can go wrong (partial warps and tiles, runs that change row of cells, lists beyond a stage,
+crowded cells, the edges between two routes) against the CPU oracle, and the one-launch step
+loop against the host loop of separate kernels bit for bit."""
 import numpy as np
 import pytest
 
@@ -91,3 +93,44 @@ def test_crowded_cells(n):
     assert g.digest() == o.digest()
     for a, b in zip(g.particles(np.arange(n)), o.particles(np.arange(n))):
         assert np.array_equal(a, b)
+
+
+def _chain_bonds(n, beads):
+    k = np.arange(n - 1)
+    k = k[(k + 1) % beads != 0]
+    return np.stack([k, k + 1], 1)
+
+
+# sizes around the edges of the one-launch loop's rules: one block, partial blocks, 4 and 2
+# lanes a particle (23,000 and 37,000), the last size it takes and the first it does not
+@pytest.mark.parametrize("prec,shape,types,fene", [
+    (_abi.PREC_FP64, (11, 11, 11), 1, False), (_abi.PREC_MIXED, (11, 11, 11), 2, False),
+    (_abi.PREC_MIXED, (13, 13, 12), 1, False), (_abi.PREC_FP64, (28, 28, 29), 1, False),
+    (_abi.PREC_FP64, (28, 29, 29), 2, False), (_abi.PREC_MIXED, (33, 33, 33), 1, False),
+    (_abi.PREC_MIXED, (33, 33, 35), 1, False), (_abi.PREC_FP64, (36, 36, 36), 1, False),
+    (_abi.PREC_FP64, (36, 36, 37), 1, False), (_abi.PREC_MIXED, (40, 40, 40), 1, False),
+    (_abi.PREC_MIXED, (41, 40, 40), 2, False), (_abi.PREC_MIXED, (20, 20, 25), 1, True),
+    (_abi.PREC_FP64, (20, 20, 25), 1, True)])
+def test_step_loop_matches_host_loop(prec, shape, types, fene, monkeypatch):
+    pos, box = _box_lattice(*shape, rho=0.85 if fene else RHO, seed=3)
+    n = len(pos)
+    typ = (np.random.default_rng(2).random(n) < 0.3).astype(np.int32) if types == 2 else None
+    vel = mb_velocities(n, 1.2, 5)
+    sims = []
+    for graph in ("0", "1"):
+        monkeypatch.setenv("ESPP_B200_GRAPH", graph)
+        s = _fluid(cuda_lib(), prec, pos, box, typ, vel)
+        if fene:
+            # bonds of lattice neighbours along x, 1.06 long
+            b = _chain_bonds(n, shape[0])
+            s.bonds(b)
+            s.fene(30.0, 0.0, 1.5)
+        s.langevin(1.0, 1.2)
+        for steps in (1, 23, 6):
+            s.run(steps)
+        sims.append(s)
+    a, b = (s.particles(np.arange(n)) for s in sims)
+    for x, y in zip(a, b):
+        assert np.array_equal(x, y)
+    assert sims[0].num_resorts() == sims[1].num_resorts()
+    assert sims[0].builds() == sims[1].builds()
