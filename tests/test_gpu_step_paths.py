@@ -3,10 +3,13 @@ observable kernel runs depends on sizes, types and density.  Each route at the s
 can go wrong (partial warps and tiles, runs that change row of cells, lists beyond a stage,
 crowded cells, the edges between two routes) against the CPU oracle, and the one-launch step
 loop against the host loop of separate kernels bit for bit."""
+import ctypes
+
 import numpy as np
 import pytest
 
 from espressopp_b200 import _abi
+from espressopp_b200._abi import call, dptr
 from simdriver import Sim, cell_grid, cuda_lib, mb_velocities, oracle_lib
 
 pytestmark = pytest.mark.gpu
@@ -134,3 +137,27 @@ def test_step_loop_matches_host_loop(prec, shape, types, fene, monkeypatch):
         assert np.array_equal(x, y)
     assert sims[0].num_resorts() == sims[1].num_resorts()
     assert sims[0].builds() == sims[1].builds()
+
+
+@pytest.mark.parametrize("bins", [1, 7, 256, 1025, 8192, 8193, 12000])
+@pytest.mark.parametrize("shape", [(11, 12, 13), (16, 16, 16)])
+def test_rdf_counts(bins, shape):
+    """Integer counts times one factor: equal to the oracle's in every bin."""
+    pos, box = _box_lattice(*shape, jitter=0.3, seed=bins)
+    out = []
+    for lib in (cuda_lib(), oracle_lib()):
+        s = Sim(lib, box, SKIN, cell_grid(box, RC, SKIN), seed=3)
+        s.add(np.arange(len(pos)), pos)
+        s.decompose()
+        g = np.zeros(bins)
+        call(lib, "espp_rdf", s.h, bins, dptr(g))
+        # positions outside the box, half a box and more: one shift is not the minimum image
+        far = pos[:40] + box * np.random.default_rng(1).uniform(-0.9, 0.9, (40, 3))
+        ids = np.arange(40, dtype=np.int64)
+        call(lib, "espp_set_particles", s.h, 40, ids.ctypes.data_as(
+            ctypes.POINTER(ctypes.c_int64)), dptr(np.ascontiguousarray(far)), None)
+        h = np.zeros(bins)
+        call(lib, "espp_rdf", s.h, bins, dptr(h))
+        out.append((g, h))
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
