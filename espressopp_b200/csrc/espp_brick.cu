@@ -904,7 +904,7 @@ void launch_lj_observables_brick(const DevView& d, double* partials, int nblocks
   const size_t sm = brick_smem_f64(d.brick.wmax);
   allow_smem(k_lj_obs_brick, sm, st);
   k_lj_obs_brick<<<d.brick.nbricks, kBrickThreads, sm, st>>>(d, energy, partials);
-  k_sum_partials<7><<<1, 256, 0, st>>>(partials, d.brick.nbricks, out);
+  k_sum_partials<7><<<1, kSumThreads, 0, st>>>(partials, d.brick.nbricks, out);
 }
 
 void launch_pair_count_brick(const DevView& d, int32_t* counts, cudaStream_t st) {

@@ -252,25 +252,32 @@ __device__ void block_sum_store(double (&v)[NV], double* partials) {
   }
 }
 
-// Fixed-order sum of the block partials (one block) -> out[0..NV)
+// Fixed-order sum of the block partials (one block of kSumThreads) -> out[0..NV)
+constexpr int kSumThreads = 1024;
 template <int NV>
-__global__ void k_sum_partials(const double* __restrict__ partials, int nblocks, double* out) {
-  __shared__ double sm[NV][256];
+__global__ void __launch_bounds__(kSumThreads) k_sum_partials(const double* __restrict__ partials,
+                                                              int nblocks, double* out) {
+  __shared__ double sm[NV][kSumThreads / 32];
   double acc[NV];
 #pragma unroll
   for (int c = 0; c < NV; ++c) acc[c] = 0.0;
-  for (int b = threadIdx.x; b < nblocks; b += blockDim.x)
+  for (int b = threadIdx.x; b < nblocks; b += kSumThreads)
 #pragma unroll
     for (int c = 0; c < NV; ++c) acc[c] += partials[(size_t)b * NV + c];
 #pragma unroll
-  for (int c = 0; c < NV; ++c) sm[c][threadIdx.x] = acc[c];
+  for (int c = 0; c < NV; ++c) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
+    if ((threadIdx.x & 31) == 0) sm[c][threadIdx.x >> 5] = acc[c];
+  }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < 32) {
 #pragma unroll
     for (int c = 0; c < NV; ++c) {
-      double t = 0.0;
-      for (int w = 0; w < (int)blockDim.x; ++w) t += sm[c][w];
-      out[c] = t;
+      double t = sm[c][threadIdx.x];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if (threadIdx.x == 0) out[c] = t;
     }
   }
 }
