@@ -953,15 +953,18 @@ constexpr double kApartMs = 0.006;
 void launch_all_forces(espp_system* s, cudaStream_t st) {
   DevView d = s->view();
   const bool mixed = s->precision == ESPP_PREC_MIXED;
-  DevView dm = d;
+  if (!s->has_vl) d.tabNT = 0;
+  // with neither LJ pairs nor FENE bonds the tabulated pass writes the forces itself
+  const bool lj = s->has_vl && s->lj_any;
+  const bool main = s->brickOn || lj || s->fene.on || !has_tab_forces(d);
   if (s->brickOn) {
     launch_forces_brick(d, mixed, s->fene, st);
-  } else {
-    if (!s->has_vl || !s->lj_any) dm.nn = s->nnZero;  // no LJ term: bonds only
+  } else if (main) {
+    DevView dm = d;
+    if (!lj) dm.nn = s->nnZero;  // no LJ term: bonds only
     launch_forces(dm, mixed, s->fene, force_tpp(s), st);
   }
-  if (!s->has_vl) d.tabNT = 0;
-  launch_force_tab(d, mixed, st);
+  launch_force_tab(d, mixed, main, st);
   if (d.mlp.on) launch_mlp_forces(d, mixed, nullptr, st);
   launch_angle_forces(d, mixed, st);
 }

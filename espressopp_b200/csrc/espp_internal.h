@@ -268,8 +268,9 @@ void launch_angle_forces(const DevView& d, bool mixed, cudaStream_t st);
 // kind 0: interaction::Cosine, 1: TabulatedAngular
 void launch_angle_observables(const DevView& d, double* partials, int nblocks, double* out,
                               int energy, int kind, cudaStream_t st);
-// tabulated pair and bond forces, added to the main kernel's output
-void launch_force_tab(const DevView& d, bool mixed, cudaStream_t st);
+// tabulated pair and bond forces, added to the main kernel's output (add) or written
+inline bool has_tab_forces(const DevView& d) { return d.tabNT > 0 || d.tabBond >= 0; }
+void launch_force_tab(const DevView& d, bool mixed, bool add, cudaStream_t st);
 void launch_tab_observables(const DevView& d, int bond, double* partials, int nblocks,
                             double* out, int energy, cudaStream_t st);
 void launch_kinetic(const DevView& d, double* partials, int nblocks, double* out,

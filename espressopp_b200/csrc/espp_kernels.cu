@@ -2171,62 +2171,115 @@ __device__ __forceinline__ double tab_dist(const DevView& d, const double* X, in
 // Tabulated pair forces over the Verlet list (VerletListTabulated: force = dist *
 // getForce(r) / r below the cutoff, Tabulated.hpp:99-115) and tabulated bond forces
 // over the fixed pair list (FixedPairListTabulated), added to the forces the main pair
-// kernel wrote.  One thread per particle; FP64 distances and table arithmetic in both
-// precision modes (the mixed mode adds the sum as int64 2^-32 fixed point).
-template <bool MIXED>
-__global__ void k_force_tab(DevView d) {
+// kernel wrote, or written where there is none (ADD false).  kTabLanes lanes a particle share
+// its list and its bonds: one lane a particle left 50,000 sites' chains of square root, table
+// lookup and division at 340 threads an SM (36 us); the reciprocal root serves the distance
+// and the division: 17.8 us.  FP64 distances and table arithmetic in both precision modes (the
+// mixed mode adds the sum as int64 2^-32 fixed point).
+constexpr int kTabLanes = 4;
+
+template <bool MIXED, bool ADD>
+__global__ void __launch_bounds__(256, 3) k_force_tab(DevView d) {
   const ParticleArrays a = d.pa[0];
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= d.n) return;
+  const int gt = blockIdx.x * blockDim.x + threadIdx.x, sub = gt % kTabLanes;
+  const bool act = gt / kTabLanes < d.n;  // every lane stays for the vote and the shuffles
+  const int i = act ? gt / kTabLanes : 0;
   const double* X = a.x;
-  double fx = 0.0, fy = 0.0, fz = 0.0;
-  auto add = [&](int t, int j) {
-    const TabDesc& T = d.tabs[t];
-    double dx, dy, dz;
-    const double r2 = tab_dist(d, X, i, j, dx, dy, dz);
+  const size_t c = d.cap;
+  const double xi = X[i], yi = X[c + i], zi = X[2 * c + i];
+  double f[3] = {0.0, 0.0, 0.0};
+  auto add = [&](const TabDesc T, double dx, double dy, double dz) {
+    const double r2 =
+        __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
     if (r2 > T.rcsq) return r2;
-    const double r = sqrt(r2);
-    const double ff = tab_value(T, d.tabCoef, true, r) / r;
-    fx += dx * ff;
-    fy += dy * ff;
-    fz += dz * ff;
+    const double inv = pair_rsqrt(r2);
+    double r = r2 * inv;
+    r = fma(0.5 * inv, fma(-r, r, r2), r);  // to the last bit or its neighbour
+    const double ff = tab_value(T, d.tabCoef, true, r) * inv;
+    f[0] += dx * ff;
+    f[1] += dy * ff;
+    f[2] += dz * ff;
     return r2;
   };
   if (d.tabNT > 0) {
+    using Share = ListShare<kTabLanes>;
     const int ti = a.type[i];
-    const int cnt = d.nn[i];
-    for (int k = 0; k < cnt; ++k) {
-      const int j = d.nl[nl_index(k, i, d.cap)];
-      const int tj = a.type[j];
-      if (ti >= d.tabNT || tj >= d.tabNT) continue;
-      const int t = d.tabPair[ti * d.tabNT + tj];
-      if (t >= 0) add(t, j);
-    }
+    const int32_t* const row = ti < d.tabNT ? d.tabPair + ti * d.tabNT : nullptr;
+    const bool single = d.tabNT == 1 && d.tabPair[0] >= 0;  // one type pair: one descriptor
+    const TabDesc T0 = d.tabs[single ? d.tabPair[0] : 0];
+    auto loop = [&](auto wrap, auto one) {
+      constexpr bool ONE = decltype(one)::value;
+      Share::walk(d, i, sub, act && row ? d.nn[i] : 0, [&](const int (&j)[Share::ENT], auto next) {
+        double xj[Share::ENT], yj[Share::ENT], zj[Share::ENT];
+        int tj[Share::ENT];
+#pragma unroll
+        for (int u = 0; u < Share::ENT; ++u) {
+          xj[u] = __ldg(&X[j[u]]);
+          yj[u] = __ldg(&X[c + j[u]]);
+          zj[u] = __ldg(&X[2 * c + j[u]]);
+          tj[u] = ONE ? 0 : __ldg(&a.type[j[u]]);
+        }
+        next();
+#pragma unroll
+        for (int u = 0; u < Share::ENT; ++u) {
+          // padding entries are the particle itself
+          int t = -1;
+          if (ONE)
+            t = j[u] != i ? 0 : -1;
+          else if (j[u] != i && tj[u] < d.tabNT)
+            t = row[tj[u]];
+          if (t < 0) continue;
+          double dx = xi - xj[u], dy = yi - yj[u], dz = zi - zj[u];
+          if (decltype(wrap)::value) {
+            dx = min_image(dx, d.L[0], d.halfL[0]);
+            dy = min_image(dy, d.L[1], d.halfL[1]);
+            dz = min_image(dz, d.L[2], d.halfL[2]);
+          }
+          if constexpr (ONE)
+            add(T0, dx, dy, dz);
+          else
+            add(d.tabs[t], dx, dy, dz);
+        }
+      });
+    };
+    const double m = d.wrapMargin;
+    const bool inner = xi > m && xi < d.L[0] - m && yi > m && yi < d.L[1] - m && zi > m &&
+                       zi < d.L[2] - m;
+    // every lane of a warp takes the same branch
+    const bool in = __all_sync(0xffffffffu, inner || !act) != 0;
+    if (single)
+      in ? loop(std::false_type{}, std::true_type{}) : loop(std::true_type{}, std::true_type{});
+    else
+      in ? loop(std::false_type{}, std::false_type{}) : loop(std::true_type{}, std::false_type{});
   }
-  if (d.tabBond >= 0 && d.bondStart) {
+  if (act && d.tabBond >= 0 && d.bondStart) {
     const int64_t off = a.id[i] - d.idMin;
-    const int b0 = d.bondStart[off], b1 = d.bondStart[off + 1];
+    const int b0 = d.bondStart[off] + sub, b1 = d.bondStart[off + 1];
     double bmax = 0.0;
-    for (int b = b0; b < b1; ++b) {
+    for (int b = b0; b < b1; b += kTabLanes) {
       const int64_t po = d.bondPartner[b] - d.idMin;
       const int j = (po >= 0 && po < d.idSpan) ? d.id2idx[po] : -1;
       if (j < 0) {
         atomicOr(d.err, kErrBondMissing);
         continue;
       }
-      bmax = fmax(bmax, add(d.tabBond, j));
+      bmax = fmax(bmax, add(d.tabs[d.tabBond], min_image(xi - X[j], d.L[0], d.halfL[0]),
+                            min_image(yi - X[c + j], d.L[1], d.halfL[1]),
+                            min_image(zi - X[2 * c + j], d.L[2], d.halfL[2])));
     }
     if (b1 > b0) note_bond_sq(d.ctr, bmax);
   }
-  const size_t c = d.cap;
-  if (MIXED) {
-    d.ffix[i] += to_fix_d(fx, d.err);
-    d.ffix[c + i] += to_fix_d(fy, d.err);
-    d.ffix[2 * c + i] += to_fix_d(fz, d.err);
-  } else {
-    d.f64[i] += fx;
-    d.f64[c + i] += fy;
-    d.f64[2 * c + i] += fz;
+#pragma unroll
+  for (int o = kTabLanes / 2; o > 0; o >>= 1)
+#pragma unroll
+    for (int q = 0; q < 3; ++q) f[q] += __shfl_xor_sync(0xffffffffu, f[q], o, kTabLanes);
+  if (!act || sub != 0) return;
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    if (MIXED)
+      d.ffix[q * c + i] = to_fix_d(f[q], d.err) + (ADD ? d.ffix[q * c + i] : 0ll);
+    else
+      d.f64[q * c + i] = ADD ? d.f64[q * c + i] + f[q] : f[q];
   }
 }
 
@@ -2788,12 +2841,15 @@ void launch_angle_observables(const DevView& d, double* partials, int nblocks, d
   k_sum_partials<7><<<1, kSumThreads, 0, st>>>(partials, nblocks, out);
 }
 
-void launch_force_tab(const DevView& d, bool mixed, cudaStream_t st) {
-  if (d.n == 0 || (d.tabNT == 0 && d.tabBond < 0)) return;
+void launch_force_tab(const DevView& d, bool mixed, bool add, cudaStream_t st) {
+  if (d.n == 0 || !has_tab_forces(d)) return;
+  const int nb = blocks_for((long long)d.n * kTabLanes);
   if (mixed)
-    k_force_tab<true><<<blocks_for(d.n), kBlock, 0, st>>>(d);
+    add ? k_force_tab<true, true><<<nb, kBlock, 0, st>>>(d)
+        : k_force_tab<true, false><<<nb, kBlock, 0, st>>>(d);
   else
-    k_force_tab<false><<<blocks_for(d.n), kBlock, 0, st>>>(d);
+    add ? k_force_tab<false, true><<<nb, kBlock, 0, st>>>(d)
+        : k_force_tab<false, false><<<nb, kBlock, 0, st>>>(d);
 }
 
 void launch_tab_observables(const DevView& d, int bond, double* partials, int nblocks,

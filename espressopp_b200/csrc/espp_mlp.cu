@@ -98,13 +98,28 @@ __device__ __forceinline__ void rbf_rec(const MlpDev& m, float r, float inv_dmu,
 
 // Pair vector d = x_i - x_j from the box-wrapped int32 coordinates (the minimum image is
 // the 32-bit wrap of the exact integer difference) and r^2 in FP32.
-__device__ __forceinline__ float pair_q(const DevView& d, const int4 pi, int j, float& dx,
+__device__ __forceinline__ float pair_q(const DevView& d, const int4 pi, const int4 pj, float& dx,
                                         float& dy, float& dz) {
-  const int4 pj = __ldg(&d.posq[j]);
   dx = wrapped_diff(pi.x, pj.x, d.fixUnit[0]);
   dy = wrapped_diff(pi.y, pj.y, d.fixUnit[1]);
   dz = wrapped_diff(pi.z, pj.z, d.fixUnit[2]);
   return fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+}
+
+// Visits the list partners of site i that fall to lane sub of its kMlpTpp: f(j, packed
+// coordinates of j), the coordinates of a step's partners loaded together and ahead of them
+// (one at a time, a site's 32 partners were as many round trips to L2).
+template <class F>
+__device__ __forceinline__ void mlp_partners(const DevView& d, int i, int sub, int cnt, F&& f) {
+  using Share = ListShare<kMlpTpp>;
+  Share::walk(d, i, sub, cnt, [&](const int (&j)[Share::ENT], auto next) {
+    int4 q[Share::ENT];
+#pragma unroll
+    for (int u = 0; u < Share::ENT; ++u) q[u] = __ldg(&d.posq[j[u]]);
+    next();
+#pragma unroll
+    for (int u = 0; u < Share::ENT; ++u) f(j[u], q[u]);
+  });
 }
 
 // G_i = sum_j g(r_ij) over the list partners within rc.
@@ -120,12 +135,10 @@ __global__ void k_mlp_desc(DevView d) {
   float G[K];
 #pragma unroll
   for (int k = 0; k < K; ++k) G[k] = 0.f;
-  const int cnt = act ? d.nn[i] : 0;
-  for (int q = sub; q < cnt; q += kMlpTpp) {
-    const int j = d.nl[nl_index(q, i, d.cap)];
+  mlp_partners(d, i, sub, act ? d.nn[i] : 0, [&](int j, const int4 pj) {
     float dx, dy, dz;
-    const float r2 = pair_q(d, pi, j, dx, dy, dz);
-    if (!(r2 < rc2) || j == i) continue;
+    const float r2 = pair_q(d, pi, pj, dx, dy, dz);
+    if (!(r2 < rc2) || j == i) return;
     float g[K];
     if (FAST)
       rbf_rec(m, sqrtf(r2), inv_dmu, g, nullptr);
@@ -133,7 +146,7 @@ __global__ void k_mlp_desc(DevView d) {
       rbf<false>(m, sqrtf(r2), g, nullptr);
 #pragma unroll
     for (int k = 0; k < K; ++k) G[k] += g[k];
-  }
+  });
 #pragma unroll
   for (int k = 0; k < K; ++k) G[k] = tpp_sum(G[k]);
   if (act && sub == 0) {
@@ -225,12 +238,10 @@ __global__ void k_mlp_force(DevView d, float* fout) {
 #pragma unroll
   for (int k = 0; k < K; ++k) Di[k] = m.D[(size_t)i * K + k];
   float fx = 0.f, fy = 0.f, fz = 0.f;
-  const int cnt = act ? d.nn[i] : 0;
-  for (int q = sub; q < cnt; q += kMlpTpp) {
-    const int j = d.nl[nl_index(q, i, d.cap)];
+  mlp_partners(d, i, sub, act ? d.nn[i] : 0, [&](int j, const int4 pj) {
     float dx, dy, dz;
-    const float r2 = pair_q(d, pi, j, dx, dy, dz);
-    if (!(r2 < rc2) || j == i) continue;
+    const float r2 = pair_q(d, pi, pj, dx, dy, dz);
+    if (!(r2 < rc2) || j == i) return;
     const float r = sqrtf(r2);
     float gp[K];
     if (FAST)
@@ -249,7 +260,7 @@ __global__ void k_mlp_force(DevView d, float* fout) {
     fx -= s * dx;
     fy -= s * dy;
     fz -= s * dz;
-  }
+  });
   fx = tpp_sum(fx);
   fy = tpp_sum(fy);
   fz = tpp_sum(fz);
@@ -333,12 +344,10 @@ __global__ void k_mlp_vpass(DevView d, const float* err, float* tangent) {
   float v[K];
 #pragma unroll
   for (int k = 0; k < K; ++k) v[k] = 0.f;
-  const int cnt = act ? d.nn[i] : 0;
-  for (int q = sub; q < cnt; q += kMlpTpp) {
-    const int j = d.nl[nl_index(q, i, d.cap)];
+  mlp_partners(d, i, sub, act ? d.nn[i] : 0, [&](int j, const int4 pj) {
     float dx, dy, dz;
-    const float r2 = pair_q(d, pi, j, dx, dy, dz);
-    if (!(r2 < rc2) || j == i) continue;
+    const float r2 = pair_q(d, pi, pj, dx, dy, dz);
+    if (!(r2 < rc2) || j == i) return;
     const float r = sqrtf(r2);
     float gp[K];
     if (FAST)
@@ -349,7 +358,7 @@ __global__ void k_mlp_vpass(DevView d, const float* err, float* tangent) {
                         (ez - err[3 * (size_t)j + 2]) * dz) / r;
 #pragma unroll
     for (int k = 0; k < K; ++k) v[k] += gp[k] * proj;
-  }
+  });
 #pragma unroll
   for (int k = 0; k < K; ++k) v[k] = tpp_sum(v[k]);
   if (act && sub == 0) {
