@@ -68,6 +68,13 @@ void dfree(T*& p) {
   p = nullptr;
 }
 
+// pinned host mirror of what a run reads back
+struct HostState {
+  DevCounters ctr;
+  unsigned err;
+  ParticleArrays pa[2];
+};
+
 }  // namespace
 
 struct espp_system {
@@ -134,6 +141,7 @@ struct espp_system {
   unsigned* err = nullptr;
   DevCounters* ctr = nullptr;     // device
   DevCounters* hctr = nullptr;    // pinned host mirror
+  HostState* hstate = nullptr;    // pinned
   ParticleArrays* d_pa = nullptr; // device: [0] current, [1] re-sort target
   bool paHostValid = true;        // host A/B mirror what d_pa holds
   double* obs = nullptr;
@@ -606,8 +614,7 @@ unsigned read_err(espp_system* s) {
   return e;
 }
 
-void check_err(espp_system* s) {
-  unsigned e = read_err(s);
+void raise_err(espp_system* s, unsigned e) {
   if (!e) return;
   cuda_check(cudaMemsetAsync(s->err, 0, sizeof(unsigned), s->st), "memset");
   if (e & kErrOutside)
@@ -619,6 +626,8 @@ void check_err(espp_system* s) {
   if (e & kErrNlOverflow) raise(ESPP_EOVERFLOW, "Verlet list capacity exceeded");
   if (e & kErrTimeout) raise(ESPP_ETIMEOUT, "a bounded wait inside a kernel ran out");
 }
+
+void check_err(espp_system* s) { raise_err(s, read_err(s)); }
 
 // Re-sort the particles by cell (fold = Storage::decompose semantics).
 void bin(espp_system* s, bool fold) {
@@ -1068,6 +1077,27 @@ DevCounters get_counters(espp_system* s) {
   return *s->hctr;
 }
 
+// Counters, error word and the current arrays' pointers in one round trip.
+struct RunState {
+  DevCounters ctr;
+  unsigned err;
+};
+
+RunState fetch_state(espp_system* s) {
+  HostState* h = s->hstate;
+  cuda_check(cudaMemcpyAsync(&h->ctr, s->ctr, sizeof(h->ctr), cudaMemcpyDeviceToHost, s->st),
+             "counters");
+  cuda_check(cudaMemcpyAsync(&h->err, s->err, sizeof(h->err), cudaMemcpyDeviceToHost, s->st),
+             "error word");
+  cuda_check(cudaMemcpyAsync(h->pa, s->d_pa, sizeof(h->pa), cudaMemcpyDeviceToHost, s->st),
+             "arrays");
+  sync(s);
+  s->A = h->pa[0];
+  s->B = h->pa[1];
+  s->paHostValid = true;
+  return {h->ctr, h->err};
+}
+
 void destroy_graph(espp_system* s) {
   if (s->graphExec) cudaGraphExecDestroy(s->graphExec);
   if (s->graph) cudaGraphDestroy(s->graph);
@@ -1225,9 +1255,8 @@ int K_high_water(espp_system* s) { return get_counters(s).nnMax; }
 // position of an entry in either list form does not depend on the capacity (block k of
 // row i sits at (k * rows + i) * 8), so the current lists are copied into the larger
 // buffer and stay valid: no rebuild, which the reference would not do either.
-void maybe_grow_K(espp_system* s) {
+void maybe_grow_K(espp_system* s, int hw) {
   if (!s->has_vl) return;
-  const int hw = K_high_water(s);
   if (s->brickOn) {
     if (hw * 10 <= s->bKb * 9) return;
     const int Kn = (hw * 3 / 2 + 15) / 8 * 8;
@@ -1266,7 +1295,9 @@ void ensure_list_form(espp_system* s) {
 // VelocityVerlet.cpp:63-103): re-sort if flagged, lists, device counters, and the
 // start-of-run force with the Langevin heat-up factor followed by integrate1 of step 0.
 // Returns the integrate arguments of the loop.
-IntegrateArgs run_prologue(espp_system* s, int64_t nsteps, double& tResort) {
+// known: the device counters, when the caller has just read them.
+IntegrateArgs run_prologue(espp_system* s, int64_t nsteps, double& tResort,
+                           const DevCounters* known = nullptr) {
   s->nResorts = 0;
   if (!s->runBeg) {
     cuda_check(cudaEventCreate(&s->runBeg), "event");
@@ -1275,6 +1306,10 @@ IntegrateArgs run_prologue(espp_system* s, int64_t nsteps, double& tResort) {
   }
   cuda_check(cudaEventRecord(s->runBeg, s->st), "event");
   if (s->idDirty) rebuild_id_tables(s);
+  // nothing below touches the counters when neither a re-sort nor a list build is due
+  if (s->resortFlag || !s->binned ||
+      (s->has_vl && !(s->listValid && brick_wanted(s) == s->brickOn)))
+    known = nullptr;
   if (s->resortFlag) {
     double tr = now_s();
     timed_decompose(s);
@@ -1288,7 +1323,7 @@ IntegrateArgs run_prologue(espp_system* s, int64_t nsteps, double& tResort) {
   if (s->has_vl && !s->listValid) build_list(s);
   ensure_list_form(s);
   IntegrateArgs a = integrate_args(s);
-  DevCounters c0 = get_counters(s);
+  DevCounters c0 = known ? *known : get_counters(s);
   c0.maxSq = 0ull;
   c0.flag = 0;
   c0.resorts = 0;
@@ -1357,8 +1392,7 @@ void run_host_loop(espp_system* s, int64_t nsteps, const IntegrateArgs& ai, doub
 }
 
 // Bookkeeping after a graph-run step loop of nsteps.
-void graph_loop_done(espp_system* s, int64_t nsteps, bool steps) {
-  DevCounters c = get_counters(s);
+void graph_loop_done(espp_system* s, int64_t nsteps, bool steps, const DevCounters& c) {
   s->step += nsteps;
   s->nResorts = c.resorts;
   s->builds += c.resorts;
@@ -1374,13 +1408,11 @@ void graph_loop_done(espp_system* s, int64_t nsteps, bool steps) {
   }
   s->phaseLaunches[kPhRebuild] += c.resorts * resort_launches(s->view());
   s->phaseLaunches[kPhList] += s->has_vl ? c.resorts : 0;
-  s->paHostValid = false;
 }
 
-void run_epilogue(espp_system* s, double t0, double tResort, bool graphDone) {
-  sync(s);
-  check_err(s);
-  maybe_grow_K(s);
+void run_epilogue(espp_system* s, double t0, double tResort, bool graphDone, const RunState& r) {
+  raise_err(s, r.err);
+  maybe_grow_K(s, r.ctr.nnMax);
   float ms = 0.f;
   cuda_check(cudaEventElapsedTime(&ms, s->runBeg, s->runEnd), "event time");
   s->lastRunMs = ms;
@@ -1404,11 +1436,10 @@ struct RunSnapshot {
 };
 
 RunSnapshot take_snapshot(espp_system* s) {
-  sync_pa(s);
+  RunSnapshot r;
+  r.ctr = fetch_state(s).ctr;
   ensure_snapshot(s);
   copy_arrays(s, s->snap, s->A);
-  RunSnapshot r;
-  r.ctr = get_counters(s);
   r.step = s->step;
   r.builds = s->builds;
   r.resortFlag = s->resortFlag;
@@ -1465,7 +1496,7 @@ void run(espp_system* s, int64_t nsteps) {
   const double t0 = now_s();
   double tResort = 0.0;
   RunSnapshot snap = take_snapshot(s);
-  IntegrateArgs ai = run_prologue(s, nsteps, tResort);
+  IntegrateArgs ai = run_prologue(s, nsteps, tResort, &snap.ctr);
   IntegrateArgs ag = graph_args(ai);
   bool steps = steps_wanted(s);
   if (steps) {
@@ -1494,15 +1525,15 @@ void run(espp_system* s, int64_t nsteps) {
   }
   cuda_check(cudaGraphLaunch(s->graphExec, s->st), "cudaGraphLaunch");
   cuda_check(cudaEventRecord(s->runEnd, s->st), "event");
-  sync(s);
-  if (read_err(s) & (kErrNlOverflow | kErrWindow)) {
+  const RunState end = fetch_state(s);
+  if (end.err & (kErrNlOverflow | kErrWindow)) {
     // back to the state before the run, a larger list, and the run again on the host loop
     recover_overflow(s, snap);
     run_host(s, nsteps);
     return;
   }
-  graph_loop_done(s, nsteps, steps);
-  run_epilogue(s, t0, tResort, true);
+  graph_loop_done(s, nsteps, steps, end.ctr);
+  run_epilogue(s, t0, tResort, true, end);
 }
 
 void run_host(espp_system* s, int64_t nsteps) {
@@ -1510,7 +1541,7 @@ void run_host(espp_system* s, int64_t nsteps) {
   double tResort = 0.0;
   IntegrateArgs ai = run_prologue(s, nsteps, tResort);
   run_host_loop(s, nsteps, ai, tResort);
-  run_epilogue(s, t0, tResort, false);
+  run_epilogue(s, t0, tResort, false, fetch_state(s));
 }
 
 }  // namespace
@@ -1555,7 +1586,7 @@ void batch_run(espp_batch* b, int64_t nsteps) {
   for (size_t r = 0; r < R; ++r) {
     espp_system* s = b->sys[r];
     snaps[r] = take_snapshot(s);
-    ags[r] = graph_args(run_prologue(s, nsteps, tRes[r]));
+    ags[r] = graph_args(run_prologue(s, nsteps, tRes[r], &snaps[r].ctr));
     key += graph_key(s, ags[r]);
     cuda_check(cudaEventRecord(b->ready[r], s->st), "event");
     cuda_check(cudaStreamWaitEvent(b->st, b->ready[r], 0), "stream wait");
@@ -1582,13 +1613,14 @@ void batch_run(espp_batch* b, int64_t nsteps) {
   b->lastMs = ms;
   for (size_t r = 0; r < R; ++r) {
     espp_system* s = b->sys[r];
-    if (read_err(s) & (kErrNlOverflow | kErrWindow)) {
+    const RunState end = fetch_state(s);
+    if (end.err & (kErrNlOverflow | kErrWindow)) {
       recover_overflow(s, snaps[r]);
       run_host(s, nsteps);
       continue;
     }
-    graph_loop_done(s, nsteps, false);
-    run_epilogue(s, t0, tRes[r], true);
+    graph_loop_done(s, nsteps, false, end.ctr);
+    run_epilogue(s, t0, tRes[r], true, end);
   }
 }
 
@@ -1731,6 +1763,7 @@ void destroy(espp_system* s) {
   if (s->runLoop) cudaEventDestroy(s->runLoop);
   if (s->runEnd) cudaEventDestroy(s->runEnd);
   if (s->hctr) cudaFreeHost(s->hctr);
+  if (s->hstate) cudaFreeHost(s->hstate);
   if (s->st) cudaStreamDestroy(s->st);
   delete s;
 }
@@ -1863,6 +1896,7 @@ int espp_system_create(const double box[3], double skin, const int32_t cell_grid
     cuda_check(cudaMemsetAsync(s->ctr, 0, sizeof(DevCounters), s->st), "memset");
     cuda_check(cudaMemsetAsync(s->d_pa, 0, 2 * sizeof(ParticleArrays), s->st), "memset");
     cuda_check(cudaMallocHost(&s->hctr, sizeof(DevCounters)), "pinned counters");
+    cuda_check(cudaMallocHost(&s->hstate, sizeof(HostState)), "pinned state");
     if (const char* g = std::getenv("ESPP_B200_GRAPH")) s->useGraph = std::atoi(g) != 0;
     if (const char* b = std::getenv("ESPP_B200_BRICK")) s->brickAllowed = std::atoi(b) != 0;
     if (const char* b = std::getenv("ESPP_B200_BRICK_BUILD")) s->brickBuild = std::atoi(b) != 0;
@@ -2653,7 +2687,7 @@ int espp_dd_run_end(espp_system* s) {
     if (!s->ddRun) raise(ESPP_ESTATE, "no decomposed run in progress");
     s->ddRun = false;
     cuda_check(cudaEventRecord(s->runEnd, s->st), "event");
-    run_epilogue(s, s->ddT0, s->ddTResort, false);
+    run_epilogue(s, s->ddT0, s->ddTResort, false, fetch_state(s));
   });
 }
 
