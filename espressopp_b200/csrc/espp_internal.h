@@ -264,7 +264,8 @@ void launch_chain_com(const double* snap, int64_t n, int M, int L, int64_t nch, 
 void launch_rdf(const DevView& d, int rdfN, double dr, unsigned long long* hist,
                 cudaStream_t st);
 // angular forces (per triple, then gathered per particle) added to the force output
-void launch_angle_forces(const DevView& d, bool mixed, cudaStream_t st);
+void launch_angle_terms(const DevView& d, cudaStream_t st);
+void launch_angle_forces(const DevView& d, bool mixed, cudaStream_t st);  // from the terms
 // kind 0: interaction::Cosine, 1: TabulatedAngular
 void launch_angle_observables(const DevView& d, double* partials, int nblocks, double* out,
                               int energy, int kind, cudaStream_t st);

@@ -2826,9 +2826,16 @@ void launch_rdf(const DevView& d, int rdfN, double dr, unsigned long long* hist,
     k_rdf<false, false><<<(unsigned)nblocks, kRdfTile, 0, st>>>(d, rdfN, (int)ntiles, dr, 1, hist);
 }
 
+static bool has_angles(const DevView& d) {
+  return d.n > 0 && d.ntriples > 0 && (d.cosine.on || d.tabAngle >= 0);
+}
+
+void launch_angle_terms(const DevView& d, cudaStream_t st) {
+  if (has_angles(d)) k_angle_forces<<<blocks_for(d.ntriples), kBlock, 0, st>>>(d);
+}
+
 void launch_angle_forces(const DevView& d, bool mixed, cudaStream_t st) {
-  if (d.n == 0 || d.ntriples == 0 || (!d.cosine.on && d.tabAngle < 0)) return;
-  k_angle_forces<<<blocks_for(d.ntriples), kBlock, 0, st>>>(d);
+  if (!has_angles(d)) return;
   if (mixed)
     k_angle_gather<true><<<blocks_for(d.n), kBlock, 0, st>>>(d);
   else

@@ -520,7 +520,6 @@ void launch_mlp_energy_terms(const DevView& d, cudaStream_t st) {
 
 void launch_mlp_forces(const DevView& d, bool mixed, float* fout, cudaStream_t st) {
   if (d.n == 0 || !d.mlp.on) return;
-  launch_mlp_energy_terms(d, st);
   const unsigned nb = (d.n * kMlpTpp + 255) / 256;
   if (mixed)
     d.mlp.tc ? k_mlp_force<true, true><<<nb, 256, 0, st>>>(d, fout)

@@ -31,10 +31,10 @@ namespace espp {
 
 MlpDev mlp_view(const espp_mlp* m);
 
-// descriptor G, site network (D = dE/dG, E) and pair forces added to the system's
-// accumulators (or written to fout, FP32 x3 per particle, when fout is set)
-void launch_mlp_forces(const DevView& d, bool mixed, float* fout, cudaStream_t st);
 void launch_mlp_energy_terms(const DevView& d, cudaStream_t st);  // G, then D and E
+// pair forces from G and D, added to the system's accumulators (or written to fout, FP32 x3
+// per particle, when fout is set)
+void launch_mlp_forces(const DevView& d, bool mixed, float* fout, cudaStream_t st);
 // force matching: ref forces (sorted order, FP64) -> error adjoint, loss partials,
 // tangent, weight-gradient partials, reduction into grad (accumulated)
 void launch_mlp_fm_grad(const DevView& d, const float* fmodel, const double* fref, float* err,
