@@ -2205,7 +2205,9 @@ __global__ void __launch_bounds__(256, 3) k_force_tab(DevView d) {
     using Share = ListShare<kTabLanes>;
     const int ti = a.type[i];
     const int32_t* const row = ti < d.tabNT ? d.tabPair + ti * d.tabNT : nullptr;
-    const bool single = d.tabNT == 1 && d.tabPair[0] >= 0;  // one type pair: one descriptor
+    // one descriptor for every pair: the table's types are those of its last change, the
+    // system's (the LJ table's) may be more by now
+    const bool single = d.tabNT == 1 && d.ntypes == 1 && d.tabPair[0] >= 0;
     const TabDesc T0 = d.tabs[single ? d.tabPair[0] : 0];
     auto loop = [&](auto wrap, auto one) {
       constexpr bool ONE = decltype(one)::value;

@@ -12,6 +12,8 @@ from simdriver import (Sim, cell_grid, cuda_lib, lattice, load_polymer40k, mb_ve
 
 pytestmark = pytest.mark.gpu
 
+RC_SOFT = 2.5
+
 
 def _rel_rms(a, b):
     return math.sqrt(np.sum((a - b) ** 2) / np.sum(b ** 2))
@@ -132,3 +134,74 @@ def test_lj_and_tabulated_on_one_verlet_list(tmp_path):
     ref = sims[0].particles(np.arange(n))
     got = sims[1].particles(np.arange(n))
     assert np.max(np.abs(got[0] - ref[0])) < 1e-9
+
+
+def _soft_table(rc, strength):
+    r = np.linspace(0.05, rc, 400)
+    x = 1.0 - r / rc
+    return r, strength * x ** 3, 3.0 * strength * x ** 2 / rc
+
+
+def _two_types(n, seed):
+    """A jittered lattice of n^3 points; every third particle has type 1."""
+    pos, box = lattice(n, 0.8442, 0.1, seed)
+    return pos, box, (np.arange(len(pos)) % 3 == 0).astype(np.int32)
+
+
+@pytest.mark.parametrize("late", [False, True])
+@pytest.mark.parametrize("prec,tol", [(_abi.PREC_FP64, 1e-12), (_abi.PREC_MIXED, 1e-8)])
+def test_partners_of_a_type_without_a_table(prec, tol, late):
+    """Only 0-0 pairs have a table; particles of type 1 are there when it is set, or come
+    later.  Mixed: each of the ~30 contributing sums rounds once to 2^-32."""
+    pos, box, typ = _two_types(12, 7)
+    ids = np.arange(len(pos))
+    out = []
+    for lib, p in ((oracle_lib(), _abi.PREC_FP64), (cuda_lib(), prec)):
+        s = Sim(lib, box, 0.3, cell_grid(box, 2.0, 0.3), precision=p, seed=5)
+        first = typ == 0 if late else typ >= 0
+        s.add(ids[first], pos[first], types=typ[first])
+        s.decompose()
+        s.vl(2.0)
+        _tab_pair(s, 0, 0, _abi.TAB_LINEAR, _soft_table(2.0, 5.0), 2.0)
+        if late:
+            s.add(ids[typ == 1], pos[typ == 1], types=typ[typ == 1])
+        s.integrator(0.002)
+        s.run(0)
+        out.append((s.particles(ids)[2], s.energy(_abi.IA_TAB_PAIR)))
+    (fo, eo), (fg, eg) = out
+    assert _rel_rms(fg, fo) < tol
+    assert np.all(fg[typ == 1] == 0.0)
+    assert abs(eg - eo) < 1e-10 * abs(eo)
+
+
+def test_types_that_migrate_into_a_domain():
+    """Two slab domains, a 0-0 table; the particles of type 1 start in the middle of one domain
+    and drift into the other, which was set up without that type."""
+    from espressopp_b200.domain import SpatialDecomposition
+
+    pos, box = lattice(16, 0.8442, 0.05, 3)
+    cg = cell_grid(box, RC_SOFT, 0.3)
+    h = box[2] / cg[2]
+    typ = ((pos[:, 2] > 1.4 * h) & (pos[:, 2] < 1.9 * h)).astype(np.int32)
+    vel = np.zeros_like(pos)
+    vel[typ == 1, 2] = 4.0
+    ids = np.arange(len(pos), dtype=np.int64)
+    r, e, f = _soft_table(RC_SOFT, 0.5)
+    one = Sim(oracle_lib(), box, 0.3, cg, precision=_abi.PREC_FP64, seed=4)
+    one.add(ids, pos, vel, typ)
+    one.decompose()
+    one.vl(RC_SOFT)
+    _tab_pair(one, 0, 0, _abi.TAB_LINEAR, (r, e, f), RC_SOFT)
+    one.integrator(0.005)
+    dd = SpatialDecomposition(box, 0.3, cg, 2, precision=_abi.PREC_FP64, seed=4, lib=cuda_lib())
+    dd.add_particles(ids, pos, vel, typ)
+    dd.decompose()
+    dd.vl_create(RC_SOFT)
+    dd.tab_pair_set(0, 0, _abi.TAB_LINEAR, r, e, f, RC_SOFT)
+    dd.integrator_set(0.005)
+    for s in (one, dd):
+        s.run(120)
+    assert np.max(one.particles(ids)[0][typ == 1, 2]) > 2.5 * h
+    (xo, _, fo, _), (xd, _, fd, _) = one.particles(ids), dd.get_particles(ids)
+    assert np.max(np.abs(fd - fo)) < 1e-9
+    assert np.max(np.abs((xd - xo + box / 2) % box - box / 2)) < 1e-9
