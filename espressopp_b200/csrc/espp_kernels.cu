@@ -19,6 +19,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "espp_device.h"
@@ -356,15 +357,38 @@ __global__ void k_xrel(DevView d) {
 
 // ---- Verlet list -------------------------------------------------------------------
 
-// Both forms of the build test the candidates of a run of particles in FP32 on coordinates
-// relative to a cell, staged in shared memory ("chunks"), two candidates per packed f32x2
-// operation, every lane against its own particle.  Candidates within the relative 2e-5 band
-// around (rc + skin)^2 are decided, after the chunk's other partners, by the reference's
-// FP64 arithmetic (exact_pair_test: d = p1 - (p2 + ghost shift), ((dx dx + dy dy) + dz dz),
-// Particle.hpp:93-98, DomainDecomposition.cpp:1347-1391).  The pair set is therefore the
-// reference's (VerletList.cpp:274-450), and each list is in a fixed order.  Lists are written
-// in whole 32-byte sectors.
+// Both forms of the build test the candidates of a group of particles in FP32 on coordinates
+// relative to the group's first cell, staged in shared memory ("chunks"), two candidates per
+// packed f32x2 operation, every lane against its own particle.  Candidates within a band
+// around (rc + skin)^2 (BuildBand) are decided, after the chunk's other partners, by the
+// reference's FP64 arithmetic (exact_pair_test: d = p1 - (p2 + ghost shift),
+// ((dx dx + dy dy) + dz dz), Particle.hpp:93-98, DomainDecomposition.cpp:1347-1391).  The pair
+// set is therefore the reference's (VerletList.cpp:274-450), and each list is in a fixed
+// order.  Lists are written in whole 32-byte sectors.
 constexpr int kStageLd = 44;  // staging row: <= 7 carried + <= 32 appended; 11 x 16 B
+
+// x-cells a group spans beyond its first one, at most: its candidate x-cells ca-h .. cb+h then
+// number 32, and the FP32 coordinates stay small enough for a narrow band.
+__host__ __device__ __forceinline__ int group_span(int h) { return 31 - 2 * h; }
+
+// The FP32 test's band.  A coordinate of up to X (the edge of a group's frame) is rounded at
+// most twice, the difference of two is off by at most 4 * 2^-24 X on an axis, and r^2 by
+// (2 q + q^2) r^2 with q = 4 * 2^-24 |(X, Y, Z)| / r, besides 3e-7 r^2 of its own rounding.
+// 2e-5 covers 31 cells as wide as the cutoff (1.5e-5); a frame of wider cells gets its own.
+struct BuildBand {
+  float lo, hi;   // FP32 decides outside
+  float mid, hw;  // a chunk with a candidate this near to mid is looked through again
+  float keepsq;   // squared distance from the group's bounding box beyond which none is a partner
+};
+BuildBand build_band(const DevView& d, double cutsq) {
+  const int h = d.hci;
+  const double X = (std::min(group_span(h), d.nc[0] - 1) + h + 1) * d.cellSize[0];
+  const double Y = (h + 1) * d.cellSize[1], Z = (h + 1) * d.cellSize[2];
+  const double q = 2.4e-7 * sqrt((X * X + Y * Y + Z * Z) / cutsq);
+  const double eps = std::max(2e-5, 3e-7 + q * (2.0 + q));
+  return {(float)(cutsq * (1.0 - eps)), (float)(cutsq * (1.0 + eps)), (float)cutsq,
+          (float)(cutsq * (1.5 * eps)), (float)(cutsq * (1.0 + 5.0 * eps))};
+}
 
 // Fast tests of one chunk (nv valid candidates) against the lane's particle.  Returns
 // whether any candidate came near the cutoff (a superset of the borderline band).
@@ -431,18 +455,17 @@ __device__ __forceinline__ void stage_flush(int* __restrict__ srow, int& pend, i
 
 // ---- Verlet build, run form ---------------------------------------------------------
 // One warp per 32 consecutive sorted particles, split where they change row of cells
-// (cy, cz); lane l holds particle g + l.  A group spans the x-cells ca..cb of one row; its
-// candidates are the particles of x-cells ca-1 .. cb+1 of the nine rows (cy+dy, cz+dz),
-// staged in the frame of cell (ca, cy, cz).  A candidate farther than the cutoff from the
-// bounding box of the group's particles cannot be a partner of any of them and is dropped
-// before it takes a slot of a chunk (ballot + prefix count), so the 32 lanes test only
-// survivors and no lane idles for lack of particles.
+// (cy, cz) or would span too many x-cells (group_span); lane l holds particle g + l.  A group
+// spans the x-cells ca..cb of one row; its candidates are the particles of x-cells ca-h .. cb+h
+// of the (2h+1)^2 rows around (cy, cz), staged in the frame of cell (ca, cy, cz).  A candidate
+// farther than the cutoff from the bounding box of the group's particles cannot be a partner
+// of any of them and is dropped before it takes a slot of a chunk (ballot + prefix count), so
+// the 32 lanes test only survivors and no lane idles for lack of particles.
 // A candidate of a farther cell (a group spans several x-cells) neither passes the test nor
 // comes near the cutoff where the particles were binned at their current positions in cells
 // whose edges all exceed the list cutoff by 0.1 %; elsewhere (STALE) each particle's own
 // neighbour cells are enforced.
 constexpr int kRunWarps = 4;
-// x-cells a group may span: its candidate x-cells ca-h .. cb+h number at most 32
 
 struct RunChunk {  // 64 slots: a scan takes 32, the rest waits for the next
   float x[64], y[64], z[64];
@@ -463,7 +486,8 @@ __device__ __forceinline__ float warp_fmax(float v) {
 }
 
 template <bool EXCL, bool STALE>
-__global__ void __launch_bounds__(kRunWarps * 32) k_build_nl_run(DevView d, double cutsq) {
+__global__ void __launch_bounds__(kRunWarps * 32) k_build_nl_run(DevView d, double cutsq,
+                                                                 BuildBand limits) {
   const ParticleArrays a = d.pa[0];
   __shared__ __align__(16) int s_stage[kRunWarps][32 * kStageLd];
   __shared__ __align__(16) RunChunk s_chunk[kRunWarps];
@@ -474,14 +498,12 @@ __global__ void __launch_bounds__(kRunWarps * 32) k_build_nl_run(DevView d, doub
   const int g = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32;
   if (g >= d.n) return;
   const unsigned full = 0xffffffffu;
-  const float lo = (float)(cutsq * (1.0 - 2e-5)), hi = (float)(cutsq * (1.0 + 2e-5));
-  const float mid = (float)cutsq, hw = (float)(cutsq * 3e-5);
-  const float keepsq = (float)(cutsq * (1.0 + 1e-4));
-  const unsigned long long mid2 = f2_pack(mid, mid);
+  const float lo = limits.lo, hi = limits.hi, hw = limits.hw, keepsq = limits.keepsq;
+  const unsigned long long mid2 = f2_pack(limits.mid, limits.mid);
   const float hx = (float)d.cellSize[0], hy = (float)d.cellSize[1], hz = (float)d.cellSize[2];
   const int nx = d.nc[0], ny = d.nc[1], nz = d.nc[2];
   const int h = d.hci, sw = 2 * h + 1;  // stencil reach and width (halfCellInt)
-  const int span = 31 - 2 * h;
+  const int span = group_span(h);
   const float4* __restrict__ xr = d.xrel;
   const int K = d.K;
   const size_t cap = d.cap;
@@ -707,12 +729,13 @@ __device__ __forceinline__ void stage_append(uint32_t& at, int j, float r2, floa
         : "memory");
 }
 
-// SPLIT: a run that changes row of cells is shared by two blocks, one for the first of its
-// groups, one (in the second half of the grid) for the others.  Where all blocks are resident
+// SPLIT: a run of several groups (row changes, or many x-cells) is shared by two blocks, one
+// for the first of its groups, one (in the second half of the grid) for the others.  Where all blocks are resident
 // at once the kernel lasts as long as its slowest block, and a block of two groups takes twice
 // the time of one; a large grid only pays for the extra blocks.
 template <bool EXCL, bool STENCIL, bool SPLIT>
-__global__ void __launch_bounds__(32 * kBlockW, 6) k_build_block(DevView d, double cutsq) {
+__global__ void __launch_bounds__(32 * kBlockW, 6) k_build_block(DevView d, double cutsq,
+                                                                BuildBand limits) {
   const ParticleArrays a = d.pa[0];
   constexpr int W = kBlockW;
   __shared__ __align__(16) BlockWarp s_w[W];
@@ -722,13 +745,11 @@ __global__ void __launch_bounds__(32 * kBlockW, 6) k_build_block(DevView d, doub
   const bool second = SPLIT && blockIdx.x >= gridDim.x / 2;
   const int g = (SPLIT ? (int)(blockIdx.x - (second ? gridDim.x / 2 : 0)) : (int)blockIdx.x) * 32;
   const unsigned full = 0xffffffffu;
-  const float lo = (float)(cutsq * (1.0 - 2e-5)), hi = (float)(cutsq * (1.0 + 2e-5));
-  const float mid = (float)cutsq, hw = (float)(cutsq * 3e-5);
-  const float keepsq = (float)(cutsq * (1.0 + 1e-4));
-  const unsigned long long mid2 = f2_pack(mid, mid);
+  const float lo = limits.lo, hi = limits.hi, hw = limits.hw, keepsq = limits.keepsq;
+  const unsigned long long mid2 = f2_pack(limits.mid, limits.mid);
   const float hx = (float)d.cellSize[0], hy = (float)d.cellSize[1], hz = (float)d.cellSize[2];
   const int nx = d.nc[0], ny = d.nc[1], nz = d.nc[2];
-  const int h = d.hci, sw = 2 * h + 1;
+  const int h = d.hci, sw = 2 * h + 1, span = group_span(h);
   const float4* __restrict__ xr = d.xrel;
   BlockWarp& sm = s_w[w];
   float* const sa = reinterpret_cast<float*>(sm.a);
@@ -754,7 +775,7 @@ __global__ void __launch_bounds__(32 * kBlockW, 6) k_build_block(DevView d, doub
     const int row = __shfl_sync(full, mrow, leader);
     const int ca = __shfl_sync(full, mcx, leader);
     const unsigned grp =
-        __ballot_sync(full, ((todo >> lane) & 1u) && mrow == row && mcx - ca <= (1 << 20));
+        __ballot_sync(full, ((todo >> lane) & 1u) && mrow == row && mcx - ca <= span);
     todo &= ~grp;
     if (SPLIT) {
       if (skip) {
@@ -2582,14 +2603,15 @@ void launch_build_nl(const DevView& d, double cutsq, bool fresh, cudaStream_t st
   bool stencil = !fresh;
   for (int k = 0; k < 3; ++k) stencil = stencil || d.cellSize[k] < rc;
   const bool excl = d.exclStart != nullptr;
+  const BuildBand band = build_band(d, cutsq);
 #define ESPP_BUILD_CASE(KERNEL, NB, NT)                                    \
   do {                                                                     \
     if (excl)                                                              \
-      stencil ? KERNEL(true, true)<<<NB, NT, 0, st>>>(d, cutsq)            \
-              : KERNEL(true, false)<<<NB, NT, 0, st>>>(d, cutsq);          \
+      stencil ? KERNEL(true, true)<<<NB, NT, 0, st>>>(d, cutsq, band)      \
+              : KERNEL(true, false)<<<NB, NT, 0, st>>>(d, cutsq, band);    \
     else                                                                   \
-      stencil ? KERNEL(false, true)<<<NB, NT, 0, st>>>(d, cutsq)           \
-              : KERNEL(false, false)<<<NB, NT, 0, st>>>(d, cutsq);         \
+      stencil ? KERNEL(false, true)<<<NB, NT, 0, st>>>(d, cutsq, band)     \
+              : KERNEL(false, false)<<<NB, NT, 0, st>>>(d, cutsq, band);   \
   } while (0)
 #define ESPP_RUN(E, S) k_build_nl_run<E, S>
 #define ESPP_BLOCK(E, S) k_build_block<E, S, false>

@@ -110,3 +110,52 @@ def test_two_cells_in_one_dimension_is_refused():
     27-cell stencil distinct); a smaller grid is refused with the reason, not built."""
     with pytest.raises(RuntimeError, match="at least 3 cells per dimension"):
         Sim(cuda_lib(), np.array([5.8, 25.0, 25.0]), SKIN, [2, 8, 8])
+
+
+def _near_cutoff_pairs(rng, n, box, rel):
+    """n points and a partner of each at |d|^2 within rel of (rc + skin)^2."""
+    a = rng.uniform(0, 1, (n, 3)) * box
+    u = rng.normal(size=(n, 3))
+    u /= np.linalg.norm(u, axis=1)[:, None]
+    d = (RC + SKIN) * np.sqrt(1.0 + rng.uniform(-rel, rel, n))
+    return np.concatenate([a, (a + u * d[:, None]) % box])
+
+
+def _same_pairs(pos, box, grid, excl=None, hci=1):
+    out = []
+    for lib in (oracle_lib(), cuda_lib()):
+        s = Sim(lib, box, SKIN, grid, precision=_abi.PREC_MIXED if lib is not oracle_lib()
+                else _abi.PREC_FP64, seed=3, half_cell_int=hci)
+        s.add(np.arange(len(pos), dtype=np.int64), pos)
+        s.decompose()
+        s.vl(RC, excl=excl)
+        first = s.digest()
+        s.vl_rebuild()  # on the cells of the re-sort
+        out.append((first, s.digest()))
+    assert out[0] == out[1]
+
+
+@pytest.mark.parametrize("excluded", [False, True])
+@pytest.mark.parametrize("hci", [1, 2])
+@pytest.mark.parametrize("per_cell", [0.03, 0.1, 1.0])
+def test_long_thin_rows(per_cell, hci, excluded):
+    """Rows of 400 list cutoffs with few particles: 32 consecutive ones lie far apart, and the
+    FP32 coordinates of a group must not grow with the row.  Pairs within 1e-4 of the
+    squared cutoff, five times the band that FP64 decides."""
+    rng = np.random.Generator(np.random.PCG64(25))
+    edge = 2.81 / hci
+    grid = [400 * hci, 2 * hci + 3, 2 * hci + 3]
+    box = np.array(grid, float) * edge
+    n = int(per_cell * box.prod() / 2.81 ** 3 / 2)
+    pos = _near_cutoff_pairs(rng, n, box, 1e-4)
+    excl = np.stack([np.arange(0, n, 2), n + np.arange(0, n, 2)], 1) if excluded else None
+    _same_pairs(pos, box, grid, excl, hci)
+
+
+@pytest.mark.parametrize("edge", [30.0, 3000.0])
+def test_cells_far_wider_than_the_cutoff(edge):
+    """Coordinates relative to a cell of many cutoffs round coarsely in FP32."""
+    rng = np.random.Generator(np.random.PCG64(26))
+    grid = [3, 4, 3]
+    box = np.array(grid, float) * edge
+    _same_pairs(_near_cutoff_pairs(rng, 700, box, 1e-4), box, grid)
