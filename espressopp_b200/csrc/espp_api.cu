@@ -105,6 +105,7 @@ struct espp_system {
   RebuildScratch scr{};
   bool binned = false;
   bool listValid = false;
+  bool runForm = false;    // too many runs outgrew the block form's stages (note_rebuilt_runs)
   bool xrelFresh = false;  // xrel written by the last gather from the current positions
 
   // staging for by-id state transfers
@@ -303,6 +304,7 @@ struct espp_system {
     d.nl = nl;
     d.nn = nn;
     d.K = K;
+    d.runForm = runForm ? 1 : 0;
     d.wrapMargin = wrap_margin();
     d.ffix = ffix;
     d.f64 = f64;
@@ -1349,6 +1351,7 @@ IntegrateArgs run_prologue(espp_system* s, int64_t nsteps, double& tResort,
   c0.maxSq = 0ull;
   c0.flag = 0;
   c0.resorts = 0;
+  c0.rebuilt = 0;
   c0.step = s->step - 1;
   c0.remaining = nsteps;
   c0.pref1 = a.pref1;
@@ -1432,9 +1435,21 @@ void graph_loop_done(espp_system* s, int64_t nsteps, bool steps, const DevCounte
   s->phaseLaunches[kPhList] += s->has_vl ? c.resorts : 0;
 }
 
+// A run of particles that the block form of the list build has to build twice makes the
+// launch last 45 us longer, and where there are many they cost their warps besides.  From one a
+// build and one in 256 runs on, the run form alone is the faster (92,000 particles, half of
+// the box at density 1.45: 125 us a build, 100 in the run form; 850,000: 1,060 and 555).  Kept
+// until particles are added.
+void note_rebuilt_runs(espp_system* s, const DevCounters& c) {
+  const int64_t runs = (s->n + 31) / 32;
+  if (s->nResorts > 0 && c.rebuilt >= s->nResorts * std::max<int64_t>(1, runs / 256))
+    s->runForm = true;
+}
+
 void run_epilogue(espp_system* s, double t0, double tResort, bool graphDone, const RunState& r) {
   raise_err(s, r.err);
   maybe_grow_K(s, r.ctr.nnMax);
+  note_rebuilt_runs(s, r.ctr);
   float ms = 0.f;
   cuda_check(cudaEventElapsedTime(&ms, s->runBeg, s->runEnd), "event time");
   s->lastRunMs = ms;
@@ -1982,6 +1997,7 @@ int espp_add_particles(espp_system* s, int64_t n, const int64_t* id, const int32
     upload_lj(s);
     s->idDirty = true;
     s->resortFlag = true;
+    s->runForm = false;
     s->K = 0;
     dfree(s->nl);
   });

@@ -89,6 +89,7 @@ struct DevCounters {
   int nnMax;                 // largest neighbour count seen by the Verlet builds
   double pref1, pref2;       // Langevin prefactors of the step loop (-gamma, sqrt(24 T gamma/dt))
   unsigned long long ltMaxBondSq;  // longest bond^2 seen by the force passes, as double bits
+  long long rebuilt;         // runs of this run's list builds that the block form built twice
 };
 
 // Pointers and scalars every kernel needs; passed by value.
@@ -159,6 +160,7 @@ struct DevView {
   int32_t* nl;            // K * cap, blocks of 8: entry (k, i) at ((k/8)*cap + i)*8 + k%8
   int32_t* nn;            // neighbour count per particle
   int K;                  // neighbour capacity
+  int runForm;            // the lists are built in the run form whatever their capacity
   double wrapMargin;      // a particle farther than this from every face of the box has no
                           // partner across one
   long long* ffix;        // 3*cap pair+bond force, int64 2^-32 fixed point (mixed)

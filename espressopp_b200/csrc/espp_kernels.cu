@@ -485,18 +485,19 @@ __device__ __forceinline__ float warp_fmax(float v) {
   return v;
 }
 
+struct RunShared {  // one warp's
+  __align__(16) int stage[32 * kStageLd];
+  RunChunk chunk;
+  int pre[33];  // prefix of the candidate x-cells' counts
+  int st[32];   // their first sorted index
+};
+
+// Lists of the particles g + lane of the lanes in todo, by one warp.
 template <bool EXCL, bool STALE>
-__global__ void __launch_bounds__(kRunWarps * 32) k_build_nl_run(DevView d, double cutsq,
-                                                                 BuildBand limits) {
+__device__ __forceinline__ void build_run(const DevView& d, double cutsq, const BuildBand& limits,
+                                          int g, unsigned todo, RunShared& sh) {
   const ParticleArrays a = d.pa[0];
-  __shared__ __align__(16) int s_stage[kRunWarps][32 * kStageLd];
-  __shared__ __align__(16) RunChunk s_chunk[kRunWarps];
-  __shared__ int s_pre[kRunWarps][33];  // prefix of the candidate x-cells' counts
-  __shared__ int s_st[kRunWarps][32];   // their first sorted index
-  const int wib = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int g = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32;
-  if (g >= d.n) return;
   const unsigned full = 0xffffffffu;
   const float lo = limits.lo, hi = limits.hi, hw = limits.hw, keepsq = limits.keepsq;
   const unsigned long long mid2 = f2_pack(limits.mid, limits.mid);
@@ -508,13 +509,11 @@ __global__ void __launch_bounds__(kRunWarps * 32) k_build_nl_run(DevView d, doub
   const int K = d.K;
   const size_t cap = d.cap;
   int* __restrict__ nl = d.nl;
-  RunChunk& ch = s_chunk[wib];
-  int* __restrict__ srow = &s_stage[wib][lane * kStageLd];
+  RunChunk& ch = sh.chunk;
+  int* __restrict__ srow = &sh.stage[lane * kStageLd];
   const int ip = g + lane;
-  const bool valid = ip < d.n;
-  const int mcell = valid ? d.pcell[ip] : 0;
+  const int mcell = (todo >> lane) & 1u ? d.pcell[ip] : 0;
   const int mcx = mcell % nx, mrow = mcell / nx;
-  unsigned todo = __ballot_sync(full, valid);
   while (todo) {
     const int leader = __ffs(todo) - 1;
     const int row = __shfl_sync(full, mrow, leader);
@@ -561,12 +560,12 @@ __global__ void __launch_bounds__(kRunWarps * 32) k_build_nl_run(DevView d, doub
           const int t = __shfl_up_sync(full, pre, o);
           if (lane >= o) pre += t;
         }
-        s_st[wib][lane] = st;
-        s_pre[wib][lane + 1] = pre;
-        if (lane == 0) s_pre[wib][0] = 0;
+        sh.st[lane] = st;
+        sh.pre[lane + 1] = pre;
+        if (lane == 0) sh.pre[0] = 0;
       }
       __syncwarp();
-      const int nrow = s_pre[wib][nxs];
+      const int nrow = sh.pre[nxs];
       const float ofy = (float)oy * hy, ofz = (float)oz * hz;
       int fill = 0;
       for (int cb0 = 0; cb0 < nrow; cb0 += 32) {
@@ -575,8 +574,8 @@ __global__ void __launch_bounds__(kRunWarps * 32) k_build_nl_run(DevView d, doub
         float cx = 0.f, cy2 = 0.f, cz2 = 0.f;
         int j = 0, k = 0;
         if (t < nrow) {
-          while (s_pre[wib][k + 1] <= t) ++k;
-          j = s_st[wib][k] + (t - s_pre[wib][k]);
+          while (sh.pre[k + 1] <= t) ++k;
+          j = sh.st[k] + (t - sh.pre[k]);
           const float4 rj = xr[j];
           cx = rj.x + (float)(k - h) * hx;
           cy2 = rj.y + ofy;
@@ -670,6 +669,16 @@ __global__ void __launch_bounds__(kRunWarps * 32) k_build_nl_run(DevView d, doub
   }
 }
 
+template <bool EXCL, bool STALE>
+__global__ void __launch_bounds__(kRunWarps * 32) k_build_nl_run(DevView d, double cutsq,
+                                                                 BuildBand limits) {
+  __shared__ RunShared s_run[kRunWarps];
+  const int g = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32;
+  if (g >= d.n) return;
+  const unsigned valid = __ballot_sync(0xffffffffu, g + (int)(threadIdx.x & 31) < d.n);
+  build_run<EXCL, STALE>(d, cutsq, limits, g, valid, s_run[threadIdx.x >> 5]);
+}
+
 // ---- Verlet build, block form --------------------------------------------------------
 // The run form with four warps on one run of 32 particles: lane l of every warp holds
 // particle g + l, and the (2h+1)^2 rows of candidate cells are shared out among the warps
@@ -687,14 +696,18 @@ constexpr int kBlockW = 4;          // warps a run
 // Particles up to which two blocks share a run (SPLIT; one block a run: 36 us at 32,768, two:
 // 33; at 241,133 137 and 142, at 4,096,000 1.97 and 2.17 ms).
 constexpr int kBuildSplit = 100000;
-constexpr int kBlockListMax = 192;  // list capacity up to which the warps' shares fit the stages
+// List capacity up to which the block form is used.  The capacity is 1.6 times the length
+// expected from the density, and 32 more: lists of 100 entries on average.
+constexpr int kBlockListMax = 192;
 
 // Warp that takes row rr of the (2h+1)^2 rows, and its stage in entries.  One cell layer: the
 // centre row, with 29 of an LJ particle's 78 partners on average and 46 at most (counted on
 // 262,144 particles; about 60 where few cells make each a third wider), alone; opposite face
 // rows together (19, at most 37: a particle near one is far from the other); the four corner
 // rows together (10, at most 30).  With 6 blocks an SM, 240 entries a lane fill its shared
-// memory.
+// memory.  Uneven densities and h > 1 share the rows out less evenly: a run with a warp whose
+// partners outgrow its stage is built again by one warp in the run form.  A system with many
+// such runs changes to that form (note_rebuilt_runs).
 __device__ __forceinline__ int block_row_owner(int rr, int h) {
   return h > 1 ? rr % kBlockW : (int)((0x313202313ull >> (4 * rr)) & 15ull);
 }
@@ -729,17 +742,26 @@ __device__ __forceinline__ void stage_append(uint32_t& at, int j, float r2, floa
         : "memory");
 }
 
+// A block whose stages do not hold its lists: one warp builds them in the run form.
+template <bool EXCL, bool STENCIL>
+__device__ __noinline__ void rebuild_run(const DevView& d, double cutsq, const BuildBand& limits,
+                                         int g, unsigned todo, int* shared) {
+  build_run<EXCL, STENCIL>(d, cutsq, limits, g, todo, *reinterpret_cast<RunShared*>(shared));
+}
+
 // SPLIT: a run of several groups (row changes, or many x-cells) is shared by two blocks, one
-// for the first of its groups, one (in the second half of the grid) for the others.  Where all blocks are resident
-// at once the kernel lasts as long as its slowest block, and a block of two groups takes twice
-// the time of one; a large grid only pays for the extra blocks.
+// for the first of its groups, one (in the second half of the grid) for the others.  Where all
+// blocks are resident at once the kernel lasts as long as its slowest block, and a block of two
+// groups takes twice the time of one; a large grid only pays for the extra blocks.
 template <bool EXCL, bool STENCIL, bool SPLIT>
-__global__ void __launch_bounds__(32 * kBlockW, 6) k_build_block(DevView d, double cutsq,
-                                                                BuildBand limits) {
+__global__ void __launch_bounds__(32 * kBlockW, 6)
+    k_build_block(const __grid_constant__ DevView d, double cutsq,
+                  const __grid_constant__ BuildBand limits) {
   const ParticleArrays a = d.pa[0];
   constexpr int W = kBlockW;
   __shared__ __align__(16) BlockWarp s_w[W];
-  __shared__ int s_stage[block_stage_start(W) * 32];
+  __shared__ __align__(16) int s_stage[block_stage_start(W) * 32];
+  static_assert(sizeof(RunShared) <= sizeof(s_stage), "the run form works in the stages");
   __shared__ int s_cnt[W][32];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool second = SPLIT && blockIdx.x >= gridDim.x / 2;
@@ -765,9 +787,8 @@ __global__ void __launch_bounds__(32 * kBlockW, 6) k_build_block(DevView d, doub
   // that leaves room for the 8 candidates tested between two checks
   const uint32_t st0 =
       (uint32_t)__cvta_generic_to_shared(s_stage + 32 * block_stage_start(w) + lane);
-  const uint32_t stLast = st0 + 128u * (block_stage_start(w + 1) - block_stage_start(w) - 9);
+  const uint32_t stLast = st0 + 128u * (block_stage_start(w + 1) - block_stage_start(w) - 8);
   uint32_t at = st0;
-  bool over = false;
   unsigned todo = __ballot_sync(full, valid), mine = todo;
   bool skip = second;  // the first group is the other block's
   while (todo) {
@@ -843,7 +864,6 @@ __global__ void __launch_bounds__(32 * kBlockW, 6) k_build_block(DevView d, doub
             stage_append<false>(at, jb, inb ? 0.f : 1.f, 0.5f, ip);
           }
         }
-        over |= at > stLast;
         at = min(at, stLast);
       }
       if (__builtin_expect(__any_sync(full, near <= hw), 0) && own && near <= hw) {
@@ -868,12 +888,7 @@ __global__ void __launch_bounds__(32 * kBlockW, 6) k_build_block(DevView d, doub
           bool in = exact_pair_test(a.x, d.cap, ip, j, fwd, wx * d.L[0], wy * d.L[1],
                                     wz * d.L[2], cutsq);
           if (EXCL && in && is_excluded(d, idi, a.id[j])) in = false;
-          if (in) {
-            if (at < stLast)
-              stage_append<false>(at, j, 0.f, 1.f, ip);
-            else
-              over = true;
-          }
+          if (in && at < stLast) stage_append<false>(at, j, 0.f, 1.f, ip);
         }
       }
     };
@@ -983,8 +998,11 @@ __global__ void __launch_bounds__(32 * kBlockW, 6) k_build_block(DevView d, doub
   if (SPLIT && mine == 0u) return;  // the whole block: a run of one group
   const bool write = (mine >> lane) & 1u;
   s_cnt[w][lane] = (int)(at - st0) >> 7;
-  if (over) atomicOr(d.err, kErrNlOverflow);
-  __syncthreads();
+  if (__syncthreads_or(at == stLast)) {  // a stage without room left
+    if (threadIdx.x == 0) atomicAdd((unsigned long long*)&d.ctr->rebuilt, 1ull);
+    if (w == 0) rebuild_run<EXCL, STENCIL>(d, cutsq, limits, g, mine, s_stage);
+    return;
+  }
   // the lists: thread (w, lane) writes the blocks w, w + W, ... of particle g + lane
   int pre[W + 1], base[W];  // base: where entry k of the list would lie in warp u's stage
   pre[0] = 0;
@@ -2594,9 +2612,8 @@ void launch_posq(const DevView& d, cudaStream_t st) {
 
 // Cells binned at the current positions (fresh) with edges 0.1 % above the list cutoff need
 // no check of a candidate's cell (see the run form); otherwise each particle's own neighbour
-// cells are enforced.  The block form's stages hold lists of up to kBlockListMax entries;
-// longer lists (a list that overflows is rebuilt with twice the capacity) take the run form,
-// which writes its lists as it goes.
+// cells are enforced.  Lists of a capacity beyond kBlockListMax, and systems whose lists do not fit the
+// block form's stages, take the run form, which writes its lists as it goes.
 void launch_build_nl(const DevView& d, double cutsq, bool fresh, cudaStream_t st) {
   if (d.n == 0) return;
   const double rc = sqrt(cutsq) * (1.0 + 1e-3) / d.hci;
@@ -2616,7 +2633,7 @@ void launch_build_nl(const DevView& d, double cutsq, bool fresh, cudaStream_t st
 #define ESPP_RUN(E, S) k_build_nl_run<E, S>
 #define ESPP_BLOCK(E, S) k_build_block<E, S, false>
 #define ESPP_BLOCK2(E, S) k_build_block<E, S, true>
-  if (d.K > kBlockListMax)
+  if (d.K > kBlockListMax || d.runForm)
     ESPP_BUILD_CASE(ESPP_RUN, blocks_for((long long)d.n, kRunWarps * 32), kRunWarps * 32);
   else if (d.n < kBuildSplit)
     ESPP_BUILD_CASE(ESPP_BLOCK2, 2 * blocks_for((long long)d.n, 32), 32 * kBlockW);

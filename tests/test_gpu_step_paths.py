@@ -4,6 +4,7 @@ can go wrong (partial warps and tiles, runs that change row of cells, lists beyo
 crowded cells, the edges between two routes) against the CPU oracle, and the one-launch step
 loop against the host loop of separate kernels bit for bit."""
 import ctypes
+import math
 
 import numpy as np
 import pytest
@@ -62,11 +63,63 @@ def test_build_pair_set(shape, excluded):
 
 @pytest.mark.parametrize("rc", [3.2, 3.6, 5.0])
 def test_long_lists(rc):
-    """Lists beyond the block form's stages (capacity above 192 entries) take the run form."""
+    """Lists of a capacity above 192 entries take the run form."""
     pos, box = _box_lattice(17, 17, 18, jitter=0.2, seed=4)
     g = _fluid(cuda_lib(), _abi.PREC_MIXED, pos, box, rc=rc)
     o = _fluid(oracle_lib(), _abi.PREC_FP64, pos, box, rc=rc)
     assert g.digest() == o.digest()
+
+
+def _uneven(nside, dense, thin, seed):
+    """A slab of density `dense` beside one of density `thin`, half the box each."""
+    L = float(nside)
+    parts = []
+    for k, rho in enumerate((dense, thin)):
+        m = [max(1, int(round(e * rho ** (1.0 / 3.0)))) for e in (L, L, L / 2)]
+        q = np.stack(np.meshgrid(*[(np.arange(c) + 0.5) / c for c in m], indexing="ij"), -1)
+        parts.append(q.reshape(-1, 3) * [L, L, L / 2] + [0, 0, k * L / 2])
+    pos = np.concatenate(parts)
+    pos += np.random.default_rng(seed).uniform(-0.08, 0.08, pos.shape)
+    return pos % L, np.full(3, L)
+
+
+@pytest.mark.parametrize("nside", [20, 48])
+def test_uneven_density_within_the_list_capacity(nside):
+    """Lists that fit their capacity although a warp's share of some does not fit its stage:
+    the reference's pairs, and no larger lists."""
+    import torch
+
+    pos, box = _uneven(nside, 1.45, 0.25, 11)
+    n = len(pos)
+    o = _fluid(oracle_lib(), _abi.PREC_FP64, pos, box)
+    cutoff = RC + SKIN
+    K = -(-(math.ceil(n / box.prod() * 4 / 3 * math.pi * cutoff ** 3 * 1.6) + 32) // 8) * 8
+    assert K <= 192
+    count = np.bincount(o.pairs().reshape(-1), minlength=n)
+    assert 130 < count.max() <= K
+    s = Sim(cuda_lib(), box, SKIN, cell_grid(box, RC, SKIN), precision=_abi.PREC_MIXED, seed=7)
+    s.add(np.arange(n), pos)
+    s.decompose()
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    s.vl(RC)
+    taken = free - torch.cuda.mem_get_info()[0]
+    assert s.digest() == o.digest()
+    assert taken < 1.5 * 4 * K * n + (4 << 20)
+    s.vl_rebuild()
+    assert s.digest() == o.digest()
+    # free flight: lists built in the loop, and after it the form that the loop's builds chose
+    vel = mb_velocities(n, 1.0, 3)
+    for q in (s, o):
+        call(q.lib, "espp_set_particles", q.h, n, np.arange(n).ctypes.data_as(
+            ctypes.POINTER(ctypes.c_int64)), None, dptr(vel))
+        call(q.lib, "espp_lj_set", q.h, 0, 0, 0.0, 1.0, RC, 0.0, 0.0)
+        q.integrator(0.002)
+    for steps in (25, 25):
+        for q in (s, o):
+            q.run(steps)
+        assert s.num_resorts() == o.num_resorts() >= 1
+        assert s.digest() == o.digest()
 
 
 def test_narrow_cells():
