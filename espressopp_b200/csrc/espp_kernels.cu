@@ -1869,10 +1869,11 @@ __global__ void k_fene_obs(DevView d, FENEParams fp, int energy, double* partial
 
 constexpr int kRdfTile = 256;
 constexpr int kRdfSmemBins = 10 * 1024;  // shared counts of a block (40 KB beside the tiles)
-// Bins up to which the FP32 pass decides enough pairs: within 2e-6 rdfN of an edge (below) lies
-// a pair in 250 at 1024 bins, one in 30 at 8192.  FP64 against FP32 first, 32,768 particles:
-// 1734 / 1052 us at 2048 bins, 1755 / 1335 at 4096, 1785 / 1749 at 8192.
-constexpr int kRdfFastBins = 8192;
+// Half width of the zone about a bin's edge, in bins, up to which the FP32 pass decides enough
+// pairs (rdf_eps at 8192 bins: one pair in 30 lies within it, one in 250 at 1024).  FP64
+// against FP32 first, 32,768 particles: 1734 / 1052 us at 2048 bins, 1755 / 1335 at 4096,
+// 1785 / 1749 at 8192.
+constexpr double kRdfFastEps = 0.0165;
 
 // Bin of a pair in the reference's arithmetic (RadialDistrF.cpp:104-129): the FP64 minimum
 // image (one shift per axis, its two comparisons), static_cast<int>(|d| / dr).
@@ -1894,16 +1895,15 @@ __device__ __forceinline__ int rdf_bin(const DevView& d, double ex, double ey, d
 // histogram does not depend on the order of the additions.
 // FAST: two partners at once in packed FP32 on the box-wrapped int32 coordinates, whose
 // 32-bit difference is the minimum image; |d| / dr comes out within eps of a bin's width
-// (six roundings of 6e-8 on a distance of up to rdfN bins; eps is five times that), and only a
-// pair within eps of a bin's edge takes the reference's FP64 arithmetic, as does a block with
-// a particle outside [-L/4, 5L/4], where one shift is not the minimum image.  17 instructions
-// a pair, all of them FP32 or integer, against 40 in FP64.
+// (rdf_eps; far = 1/2 - eps), and only a pair within eps of a bin's edge takes the reference's
+// FP64 arithmetic, as does a block with a particle outside [-L/4, 5L/4], where one shift is not
+// the minimum image.  17 instructions a pair, all of them FP32 or integer, against 40 in FP64.
 // Counts go to `copies` copies of the histogram in shared memory, a lane's copy by its bank
 // (no bank conflicts with 32), flushed with one global atomic per non-empty bin.
 // Bound by issue: a call at 32,768 particles and 256 bins took 1,617 us in FP64, now 742.
 template <bool SMEM, bool FAST>
 __global__ void __launch_bounds__(kRdfTile) k_rdf(DevView d, int rdfN, int ntiles, double dr,
-                                                  int copies, unsigned long long* hist) {
+                                                  float far, int copies, unsigned long long* hist) {
   extern __shared__ unsigned s_hist[];
   using Coord = std::conditional_t<FAST, int, double>;
   __shared__ __align__(16) Coord sx[kRdfTile], sy[kRdfTile], sz[kRdfTile];
@@ -1973,7 +1973,6 @@ __global__ void __launch_bounds__(kRdfTile) k_rdf(DevView d, int rdfN, int ntile
       const float inv = (float)(1.0 / dr);
       const float gx = d.fixUnit[0] * inv, gy = d.fixUnit[1] * inv, gz = d.fixUnit[2] * inv;
       const unsigned long long ux = f2_pack(gx, gx), uy = f2_pack(gy, gy), uz = f2_pack(gz, gz);
-      const float eps = 2e-6f * (float)rdfN;
       const float magic = 12582912.f;  // 1.5 * 2^23: adding it rounds to an integer
       const unsigned long long half = f2_pack(0.5f, 0.5f);
       const unsigned long long mb = f2_pack(magic, magic);
@@ -1994,8 +1993,8 @@ __global__ void __launch_bounds__(kRdfTile) k_rdf(DevView d, int rdfN, int ntile
         const unsigned long long rh = f2_sub(r, half), y = f2_add(rh, mb);
         const unsigned long long off = f2_sub(rh, f2_sub(y, mb));  // 1/2 off at an integer r
         int ba = __float_as_int(f2_lo(y)) - 0x4B400000, bb = __float_as_int(f2_hi(y)) - 0x4B400000;
-        if (fabsf(f2_lo(off)) > 0.5f - eps) ba = exact(t);
-        if (fabsf(f2_hi(off)) > 0.5f - eps && t + 1 < jn) bb = exact(t + 1);
+        if (fabsf(f2_lo(off)) > far) ba = exact(t);
+        if (fabsf(f2_hi(off)) > far && t + 1 < jn) bb = exact(t + 1);
         if (t >= t0) count(ba);
         if (t + 1 < jn) count(bb);
       }
@@ -2848,6 +2847,14 @@ void launch_fene_observables(const DevView& d, const FENEParams& fp, double* par
   k_sum_partials<7><<<1, kSumThreads, 0, st>>>(partials, nblocks, out);
 }
 
+// Bound on the error of |d| / dr in k_rdf's FP32 arithmetic: six roundings of 6e-8 on a distance
+// of up to rdfN bins, and the packed coordinates' unit of L / 2^32 an axis; at least 2e-6 rdfN.
+static double rdf_eps(const DevView& d, int rdfN, double dr) {
+  const double unit =
+      sqrt(d.L[0] * d.L[0] + d.L[1] * d.L[1] + d.L[2] * d.L[2]) / 4294967296.0 / dr;
+  return std::max(2e-6 * rdfN, 4e-7 * rdfN + 1.1 * unit);
+}
+
 void launch_rdf(const DevView& d, int rdfN, double dr, unsigned long long* hist,
                 cudaStream_t st) {
   if (d.n < 2) return;
@@ -2857,14 +2864,16 @@ void launch_rdf(const DevView& d, int rdfN, double dr, unsigned long long* hist,
   int copies = 1;
   while (copies < 32 && 2 * copies * rdfN <= 8192) copies *= 2;
   const size_t smem = sizeof(unsigned) * rdfN * copies;
-  if (rdfN <= kRdfFastBins)
-    k_rdf<true, true><<<(unsigned)nblocks, kRdfTile, smem, st>>>(d, rdfN, (int)ntiles, dr, copies,
-                                                                 hist);
+  const double eps = rdf_eps(d, rdfN, dr);
+  if (rdfN <= kRdfSmemBins && eps <= kRdfFastEps)
+    k_rdf<true, true><<<(unsigned)nblocks, kRdfTile, smem, st>>>(d, rdfN, (int)ntiles, dr,
+                                                                 (float)(0.5 - eps), copies, hist);
   else if (rdfN <= kRdfSmemBins)
-    k_rdf<true, false><<<(unsigned)nblocks, kRdfTile, smem, st>>>(d, rdfN, (int)ntiles, dr, copies,
-                                                                  hist);
+    k_rdf<true, false><<<(unsigned)nblocks, kRdfTile, smem, st>>>(d, rdfN, (int)ntiles, dr, 0.f,
+                                                                  copies, hist);
   else
-    k_rdf<false, false><<<(unsigned)nblocks, kRdfTile, 0, st>>>(d, rdfN, (int)ntiles, dr, 1, hist);
+    k_rdf<false, false><<<(unsigned)nblocks, kRdfTile, 0, st>>>(d, rdfN, (int)ntiles, dr, 0.f, 1,
+                                                                hist);
 }
 
 static bool has_angles(const DevView& d) {

@@ -216,6 +216,23 @@ def test_rdf_counts(bins, shape):
         assert np.array_equal(a, b)
 
 
+@pytest.mark.parametrize("ratio", [100, 2000, 30000])
+def test_rdf_counts_in_a_long_box(ratio):
+    """The bins follow the y edge; the packed coordinates of x are coarser the longer x is."""
+    rng = np.random.default_rng(ratio)
+    box = np.array([8.5 * ratio, 8.5, 8.5])
+    pos = rng.uniform(0.0, 1.0, (1500, 3)) * [8.5, 8.5, 8.5] + [0.7 * box[0], 0.0, 0.0]
+    out = []
+    for lib in (cuda_lib(), oracle_lib()):
+        s = Sim(lib, box, SKIN, cell_grid(box, RC, SKIN), seed=3)
+        s.add(np.arange(len(pos)), pos)
+        s.decompose()
+        g = np.zeros(4096)
+        call(lib, "espp_rdf", s.h, 4096, dptr(g))
+        out.append(g)
+    assert np.array_equal(*out)
+
+
 @pytest.mark.parametrize("shape", [(11, 11, 11), (17, 13, 12), (47, 47, 47)])
 @pytest.mark.parametrize("types", [1, 2])
 def test_observables(shape, types):
