@@ -1216,14 +1216,6 @@ __device__ __forceinline__ double pair_rcp(double x) {
   return fma(r, fma(e, e, e), r);
 }
 
-// 1 / sqrt(x) in the same way: y0 from the hardware, e = 1 - x y0^2, y0 (1 + e/2 + 3 e^2 / 8).
-__device__ __forceinline__ double pair_rsqrt(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-x * y, y, 1.0);
-  return fma(y * e, fma(0.375, e, 0.5), y);
-}
-
 // Plain FP64 form of the same kernel (reference arithmetic of LennardJones.hpp:137-143
 // and FENE.hpp:97-112 on minimum-image distances).  A warp whose particles all lie farther
 // than wrapMargin from every face of the box has no partner across one: its differences are
@@ -2210,10 +2202,10 @@ __device__ __forceinline__ double tab_dist(const DevView& d, const double* X, in
 // getForce(r) / r below the cutoff, Tabulated.hpp:99-115) and tabulated bond forces
 // over the fixed pair list (FixedPairListTabulated), added to the forces the main pair
 // kernel wrote, or written where there is none (ADD false).  kTabLanes lanes a particle share
-// its list and its bonds: one lane a particle left 50,000 sites' chains of square root, table
-// lookup and division at 340 threads an SM (36 us); the reciprocal root serves the distance
-// and the division: 17.8 us.  FP64 distances and table arithmetic in both precision modes (the
-// mixed mode adds the sum as int64 2^-32 fixed point).
+// its list and its bonds: one lane a particle leaves 50,000 sites' chains of square root, table
+// lookup and division at 340 threads an SM (36 us).  FP64 distances and table arithmetic, the
+// reference's operations, in both precision modes (the mixed mode adds the sum as int64 2^-32
+// fixed point).
 constexpr int kTabLanes = 4;
 
 template <bool MIXED, bool ADD>
@@ -2230,10 +2222,8 @@ __global__ void __launch_bounds__(256, 3) k_force_tab(DevView d) {
     const double r2 =
         __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
     if (r2 > T.rcsq) return r2;
-    const double inv = pair_rsqrt(r2);
-    double r = r2 * inv;
-    r = fma(0.5 * inv, fma(-r, r, r2), r);  // to the last bit or its neighbour
-    const double ff = tab_value(T, d.tabCoef, true, r) * inv;
+    const double r = sqrt(r2);
+    const double ff = tab_value(T, d.tabCoef, true, r) / r;
     f[0] += dx * ff;
     f[1] += dy * ff;
     f[2] += dz * ff;

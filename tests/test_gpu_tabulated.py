@@ -205,3 +205,28 @@ def test_types_that_migrate_into_a_domain():
     (xo, _, fo, _), (xd, _, fd, _) = one.particles(ids), dd.get_particles(ids)
     assert np.max(np.abs(fd - fo)) < 1e-9
     assert np.max(np.abs((xd - xo + box / 2) % box - box / 2)) < 1e-9
+
+
+@pytest.mark.parametrize("itype", [1, 2, 3])
+def test_force_of_dimers(itype):
+    """A single pair's FP64 force is the reference's bit for bit (Tabulated.hpp:99-115,
+    Interpolation*.hpp): every operation of dist * f(r) / r is rounded once."""
+    box = np.full(3, 9.0)
+    sims = []
+    for lib in (cuda_lib(), oracle_lib()):
+        s = Sim(lib, box, 0.3, [3, 3, 3], precision=_abi.PREC_FP64, seed=3)
+        s.add(np.arange(2), np.array([[1.0, 1.0, 1.0], [2.0, 1.0, 1.0]]))
+        s.decompose()
+        s.vl(2.0)
+        _tab_pair(s, 0, 0, itype, _soft_table(2.0, 5.0), 2.0)
+        s.integrator(0.002)
+        sims.append(s)
+    for d in np.linspace(0.3, 1.9, 150):
+        q = np.array([[1.0, 1.0, 1.0], [1.0 + 0.48 * d, 1.0 + 0.6 * d, 1.0 + 0.64 * d]])
+        f = []
+        for s in sims:
+            _abi.call(s.lib, "espp_set_particles", s.h, 2, _abi.i64ptr(np.arange(2)),
+                      _abi.dptr(q), None)
+            s.run(0)
+            f.append(s.particles(np.arange(2))[2])
+        assert np.array_equal(*f), d
