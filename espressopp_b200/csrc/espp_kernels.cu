@@ -1220,11 +1220,14 @@ __device__ __forceinline__ double pair_rcp(double x) {
 // and FENE.hpp:97-112 on minimum-image distances).  A warp whose particles all lie farther
 // than wrapMargin from every face of the box has no partner across one: its differences are
 // their own minimum images, bit for bit, and the 12 FP64 instructions of the comparisons
-// and shifts (of 30 a pair) are skipped.  The reciprocal is Newton steps on the hardware's
-// approximation instead of a division.  Bound by the FP64 pipe and the gathers: 402 us before
-// and 192 now at 1,009,091 particles (one type), 19.8 and 13 at 32,768.  Registers: four
-// blocks an SM with one type (203 us with three), three where the pair's constants are loaded
-// per entry.
+// and shifts (of 30 a pair) are skipped.  Bound by the FP64 pipe and the gathers: 186 us at a
+// million particles of one type, 13 at 32,768; with a division in place of pair_rcp 251 and 17.
+// With one or two lanes and one type a lane's entries go to two sums in turn: no sum is longer
+// than with four lanes (error against 80-bit sums 6.374e-15, 6.377e-15 with one sum,
+// 6.376e-15 with four lanes), and the chain of additions is half as long (188 us with one).
+// With several types the second sum would spill (370 us, 320 with one, at a million).
+// Registers: four blocks an SM with one type (203 us with three), three where the pair's
+// constants are loaded per entry.
 template <int T, bool SINGLE, bool CAPPED, bool FENE, bool LIVE, class Share>
 __device__ __forceinline__ void particle_force_fp64(const DevView& d, const FENEParams& fp,
                                                     const double* X, int i, int sub, bool act,
@@ -1235,8 +1238,9 @@ __device__ __forceinline__ void particle_force_fp64(const DevView& d, const FENE
   const double xi = ld_pos<LIVE>(&X[i]), yi = ld_pos<LIVE>(&Y[i]), zi = ld_pos<LIVE>(&Z[i]);
   const LJPair* const row = d.lj + (SINGLE ? 0 : a.type[i] * d.ntypes);
   const double sc1 = d.lj[0].ff1, sc2 = d.lj[0].ff2, srcsq = d.lj[0].rcsq;
-  double fx = 0, fy = 0, fz = 0;
-  auto pair = [&](double dx, double dy, double dz, int tj) {
+  constexpr int S = SINGLE && T <= 2 ? 2 : 1;  // partial sums
+  double f[S][3] = {};
+  auto pair = [&](double dx, double dy, double dz, int tj, double (&f)[3]) {
     const double r2 = dx * dx + dy * dy + dz * dz;
     const LJPair& P = row[SINGLE ? 0 : tj];
     const double c1 = SINGLE ? sc1 : P.ff1, c2 = SINGLE ? sc2 : P.ff2;
@@ -1248,9 +1252,9 @@ __device__ __forceinline__ void particle_force_fp64(const DevView& d, const FENE
     double ff = ri6 * (c1 * ri6 - c2) * ri2;
     if (CAPPED && P.caprad > 0 && !(r2 > P.caprad * P.caprad)) ff = P.capff / sqrt(r2);
     if (in) {
-      fx += dx * ff;
-      fy += dy * ff;
-      fz += dz * ff;
+      f[0] += dx * ff;
+      f[1] += dy * ff;
+      f[2] += dz * ff;
     }
   };
   auto loop = [&](auto wrap) {
@@ -1273,7 +1277,7 @@ __device__ __forceinline__ void particle_force_fp64(const DevView& d, const FENE
           dy = min_image(dy, d.L[1], d.halfL[1]);
           dz = min_image(dz, d.L[2], d.halfL[2]);
         }
-        pair(dx, dy, dz, tj[u]);
+        pair(dx, dy, dz, tj[u], f[u % S]);
       }
     });
   };
@@ -1284,6 +1288,12 @@ __device__ __forceinline__ void particle_force_fp64(const DevView& d, const FENE
     loop(std::false_type{});
   else
     loop(std::true_type{});
+  double fx = f[0][0], fy = f[0][1], fz = f[0][2];
+  if (S == 2) {
+    fx += f[S - 1][0];
+    fy += f[S - 1][1];
+    fz += f[S - 1][2];
+  }
   if (FENE && act) {
     // the particle's bonds, shared out among its lanes
     const int64_t off = a.id[i] - d.idMin;
