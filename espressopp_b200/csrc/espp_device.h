@@ -231,6 +231,15 @@ __device__ __forceinline__ long long to_fix(float f, unsigned* err) {
   return __float2ll_rn(f * 4294967296.0f);
 }
 
+// The same for a sum held in two packed partial sums, each rounded by itself: the total obeys
+// the same limit, and no partial sum leaves the range.
+__device__ __forceinline__ long long to_fix2(unsigned long long f, unsigned* err) {
+  const float a = f2_lo(f), b = f2_hi(f);
+  if (!(fabsf(a + b) < 1.0e9f) || !(fmaxf(fabsf(a), fabsf(b)) < 1.0e9f))
+    atomicOr(err, kErrFixOverflow);
+  return __float2ll_rn(a * 4294967296.0f) + __float2ll_rn(b * 4294967296.0f);
+}
+
 template <int NV>
 __device__ void block_sum_store(double (&v)[NV], double* partials) {
   __shared__ double sm[NV][kBlock / 32];

@@ -1043,7 +1043,6 @@ __global__ void __launch_bounds__(32 * kBlockW, 6)
 
 // ---- forces ------------------------------------------------------------------------
 
-constexpr int kMixMB = 4;
 // Loads of arrays that other blocks write during the kernel (LIVE) go through the coherent
 // path, others through the read-only one.
 template <bool LIVE>
@@ -1067,13 +1066,16 @@ __device__ __forceinline__ double ld_pos(const double* p) {
 // FP32 pair forces on box-wrapped int32 coordinates, T lanes a particle.  The minimum image
 // is the 32-bit wrap of the coordinate difference.  Two entries are evaluated at once in the
 // halves of packed f32x2 registers (20 instructions an entry, 31 scalar).  FP32 sums along
-// the list, the result in int64 2^-32 fixed point; the lanes' partial sums and the bond
-// terms are combined in int64, so the result does not depend on the order in which they are
-// added.  Every lane of the warp takes part (act: the lane has a particle).
+// the list, one for each half and, with one lane, two such pairs in turn, so that no FP32 sum
+// is longer than about 40 entries of a liquid's 78; each sum, the lanes' and the bond terms are
+// combined in int64 2^-32 fixed point, so the result does not depend on the order in which
+// they are added.  Every lane of the warp takes part (act: the lane has a particle).
 // Bound by the L1 data pipe: the 32 coordinates a warp gathers lie in 10 to 18 lines, 88 to 95 %
 // of the pipe's wavefronts at a million particles, issue 39 % (53 % scalar).  With ListShare
-// the lanes of a particle take adjacent entries, which share lines.  At 241,133 particles of
-// two types 59.0 us before and 46.1 now, at 32,768 11.1 and 8.1; 4,096,000 with one lane 505.
+// the lanes of a particle take adjacent entries, which share lines.  40 us at 241,133 particles
+// of two types (two lanes; 44 with the lanes on blocks of their own), 9.2 at 32,768, 495 at
+// 4,096,000 with one lane.  One lane runs three blocks an SM: with four, the second pair of
+// sums spills (526 us).
 template <int T, bool SINGLE, bool CAPPED, bool FENE, bool LIVE, class Share>
 __device__ __forceinline__ void particle_force_mixed(const DevView& d, const FENEParams& fp,
                                                      const LJPairF* sP, const int4* posq, int i,
@@ -1087,8 +1089,9 @@ __device__ __forceinline__ void particle_force_mixed(const DevView& d, const FEN
   const LJPairF P = d.ljf[0];
   const unsigned long long ff1s = f2_pack(P.ff1, P.ff1), ff2s = f2_pack(-P.ff2, -P.ff2);
   const LJPairF* const row = sP + (SINGLE ? 0 : pi.w * d.ntypes);
-  unsigned long long fx = 0ull, fy = 0ull, fz = 0ull;
-  auto pairs = [&](const int4 pa, const int4 pb) {
+  constexpr int S = T == 1 ? 2 : 1;  // pairs of FP32 sums
+  unsigned long long f[S][3] = {};
+  auto pairs = [&](const int4 pa, const int4 pb, unsigned long long (&sum)[3]) {
     const unsigned long long dx =
         f2_mul(f2_pack(wrapped_diff(pi.x, pa.x), wrapped_diff(pi.x, pb.x)), ux);
     const unsigned long long dy =
@@ -1116,10 +1119,10 @@ __device__ __forceinline__ void particle_force_mixed(const DevView& d, const FEN
     // padding entries are the particle itself: r^2 = 0
     fa = (ra > 0.f && ra <= Pa.rcsq) ? fa : 0.f;
     fb = (rb > 0.f && rb <= Pb.rcsq) ? fb : 0.f;
-    const unsigned long long f = f2_pack(fa, fb);
-    fx = f2_fma(dx, f, fx);
-    fy = f2_fma(dy, f, fy);
-    fz = f2_fma(dz, f, fz);
+    const unsigned long long fab = f2_pack(fa, fb);
+    sum[0] = f2_fma(dx, fab, sum[0]);
+    sum[1] = f2_fma(dy, fab, sum[1]);
+    sum[2] = f2_fma(dz, fab, sum[2]);
   };
   share.walk(d, i, sub, act ? d.nn[i] : 0, [&](const int (&j)[Share::ENT], auto next) {
     int4 q[Share::ENT];
@@ -1127,10 +1130,15 @@ __device__ __forceinline__ void particle_force_mixed(const DevView& d, const FEN
     for (int u = 0; u < Share::ENT; ++u) q[u] = ld_pos<LIVE>(&posq[j[u]]);
     next();
 #pragma unroll
-    for (int u = 0; u < Share::ENT; u += 2) pairs(q[u], q[u + 1]);
+    for (int u = 0; u < Share::ENT; u += 2) pairs(q[u], q[u + 1], f[u / 2 % S]);
   });
-  long long Fx = to_fix(f2_lo(fx) + f2_hi(fx), d.err), Fy = to_fix(f2_lo(fy) + f2_hi(fy), d.err),
-            Fz = to_fix(f2_lo(fz) + f2_hi(fz), d.err);
+  long long Fx = 0, Fy = 0, Fz = 0;
+#pragma unroll
+  for (int u = 0; u < S; ++u) {
+    Fx += to_fix2(f[u][0], d.err);
+    Fy += to_fix2(f[u][1], d.err);
+    Fz += to_fix2(f[u][2], d.err);
+  }
   if (FENE && act) {
     // the particle's bonds, shared out among its lanes
     const int64_t off = a.id[i] - d.idMin;
@@ -1179,7 +1187,7 @@ __device__ __forceinline__ void particle_force_mixed(const DevView& d, const FEN
 }
 
 template <int T, bool SINGLE, bool CAPPED, bool FENE>
-__global__ void __launch_bounds__(256, kMixMB) k_force_mixed(DevView d, FENEParams fp) {
+__global__ void __launch_bounds__(256, T == 1 ? 3 : 4) k_force_mixed(DevView d, FENEParams fp) {
   __shared__ LJPairF sP[kMaxTypes * kMaxTypes];
   if (!SINGLE) {
     for (int t = threadIdx.x; t < d.ntypes * d.ntypes; t += blockDim.x) sP[t] = d.ljf[t];

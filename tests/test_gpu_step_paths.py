@@ -192,6 +192,35 @@ def test_step_loop_matches_host_loop(prec, shape, types, fene, monkeypatch):
     assert sims[0].builds() == sims[1].builds()
 
 
+@pytest.mark.parametrize("tpp", [1, 2, 4, 8])
+def test_mixed_sums_are_fixed_point(tpp):
+    """FP32 partial sums are combined in 2^-32 fixed point, nothing is added in FP32 across
+    them: the force of two partners in different sums is the sum of the two forces, exactly."""
+    box = np.full(3, 12.0)
+    rng = np.random.default_rng(4)
+    s = Sim(cuda_lib(), box, SKIN, [4, 4, 4], precision=_abi.PREC_MIXED, seed=3)
+    ids = np.arange(3, dtype=np.int64)
+    s.add(ids, np.array([[6.0, 6.0, 6.0], [7.0, 6.0, 6.0], [6.0, 7.0, 6.0]]))
+    s.decompose()
+    s.vl(RC)
+    s.lj(0, 0, 1.0, 1.0, RC, SHIFT)
+    s.integrator(0.005)
+    call(s.lib, "espp_set_tpp", s.h, tpp)
+    far = np.array([11.5, 11.5, 11.5])
+    for _ in range(30):
+        u = rng.normal(size=(2, 3))
+        u /= np.linalg.norm(u, axis=1)[:, None]
+        a, b = 6.0 + u[0] * rng.uniform(0.85, 0.95), 6.0 + u[1] * rng.uniform(1.2, 2.0)
+        f = []
+        for p, q in ((a, b), (a, far), (far, b)):
+            x = np.ascontiguousarray([[6.0, 6.0, 6.0], p, q])
+            call(s.lib, "espp_set_particles", s.h, 3, ids.ctypes.data_as(
+                ctypes.POINTER(ctypes.c_int64)), dptr(x), None)
+            s.run(0)
+            f.append(s.particles(ids)[2][0])
+        assert np.array_equal(f[0], f[1] + f[2])
+
+
 @pytest.mark.parametrize("bins", [1, 7, 256, 1025, 8192, 8193, 12000])
 @pytest.mark.parametrize("shape", [(11, 12, 13), (16, 16, 16)])
 def test_rdf_counts(bins, shape):
