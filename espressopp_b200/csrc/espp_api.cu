@@ -941,15 +941,15 @@ int force_tpp(const espp_system* s) {
   if (s->tpp > 0) return s->tpp;
   // Lanes fill the GPU at small sizes and share their gathers' lines; at large ones each more
   // lane leaves fewer entries a lane.  Force pass, 1 / 2 / 4 lanes, mixed: 9.1 / 7.1 / 6.8 us at
-  // 2,028 particles, 11.2 / 9.2 / 9.2 at 32,768, 40.6 / 37.9 / 39.9 at 241,133, 131 / 136 / 159
-  // at 1,009,091, 505 / 550 / 670 at 4,096,000.  FP64, one type / two types: 16 / 13 / 13 and
+  // 2,028 particles, 11.2 / 9.2 / 9.2 at 32,768, 33.7 / 33.7 / 37.5 at 226,981, 130 / 134 / 155
+  // at a million, 495 / 548 / 659 at 4,096,000.  FP64, one type / two types: 16 / 13 / 13 and
   // 38 / 20 / 26 at 32,768, 193 / 186 / 216 and 573 / 320 / 351 at a million, 723 / 735 / 892
   // and 2170 / 1265 / 1430 at 4,096,000: one lane holds eight entries' coordinates, which
-  // spill where the constants are loaded per pair.  Below, as many as one block an SM of the
-  // step kernel has room for.
+  // spill where the constants are loaded per pair.  Four as far as the step kernel's one block
+  // an SM has room for them: with more lanes than that the steps run as separate kernels.
   const bool mixed = s->precision == ESPP_PREC_MIXED;
-  const int four = mixed ? 37000 : 23000;
-  return mixed && s->n >= 600000 ? 1 : (s->n >= four ? 2 : 4);
+  if (mixed && s->n >= 600000) return 1;
+  return 4ll * s->n <= (int64_t)s->nsm * step_threads(mixed) ? 4 : 2;
 }
 
 // Whether the steps between two re-sorts run as one cooperative launch: LJ and FENE forces
