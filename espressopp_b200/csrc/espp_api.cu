@@ -158,7 +158,7 @@ struct espp_system {
   cudaStream_t side = nullptr;
   cudaEvent_t sideBeg = nullptr, sideEnd = nullptr;
   // one-launch step loop of a small system (k_steps)
-  bool stepsOff = false;  // the cooperative launch could not be captured
+  std::string stepsRefused;  // graph key for which the GPU refused the cooperative launch
   StepSync* stepSync = nullptr;
   int4* posqAlt = nullptr;
   int posqAltCap = 0;
@@ -955,7 +955,7 @@ int force_tpp(const espp_system* s) {
 // Whether the steps between two re-sorts run as one cooperative launch: LJ and FENE forces
 // from the global list, and no more lanes than one block an SM holds.
 bool steps_wanted(const espp_system* s) {
-  return !s->stepsOff && s->n > 0 && s->n <= kStepParticles && !s->brickOn && s->tabNT == 0 &&
+  return s->n > 0 && s->n <= kStepParticles && !s->brickOn && s->tabNT == 0 &&
          s->tabBond < 0 && s->triples.empty() && !s->mlp && s->haloIds.empty() &&
          (int64_t)s->n * force_tpp(s) <=
              (int64_t)s->nsm * step_threads(s->precision == ESPP_PREC_MIXED);
@@ -1164,6 +1164,19 @@ void launch_rebuild_kernels(espp_system* s, cudaStream_t st) {
 
 void launch_force_kernel(espp_system* s, cudaStream_t st) { launch_all_forces(s, st); }
 
+// The step kernel's cooperative launch is not to be had here: the loop of separate kernels
+// takes its place.  Any other error leaves the run as an error.
+struct StepsRefused {};
+
+void steps_check(cudaError_t e, const char* what) {
+  if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported ||
+      e == cudaErrorStreamCaptureUnsupported) {
+    cudaGetLastError();
+    throw StepsRefused{};
+  }
+  cuda_check(e, what);
+}
+
 // Adds to graph g one WHILE node (no dependencies) running the step loop of s:
 // WHILE(remaining) { decide; IF(re-sort) { fold + bin, scan, scatter, sort + move, list };
 //                    force; integrate2 + integrate1 }
@@ -1205,9 +1218,9 @@ void add_step_loop(espp_system* s, cudaGraph_t g, const IntegrateArgs& ai, bool 
   if (steps) {
     DevView d = s->view();
     if (!s->has_vl || !s->lj_any) d.nn = s->nnZero;  // no LJ term: bonds only
-    cuda_check(launch_steps(d, s->precision == ESPP_PREC_MIXED, s->fene, ai, skinHalf,
-                            s->stepSync, s->posqAlt, hIf, hWhile, force_tpp(s), s->nsm, cs),
-               "step kernel");
+    steps_check(launch_steps(d, s->precision == ESPP_PREC_MIXED, s->fene, ai, skinHalf,
+                             s->stepSync, s->posqAlt, hIf, hWhile, force_tpp(s), s->nsm, cs),
+                "step kernel");
   } else {
     launch_decide_graph(s->view(), skinHalf, hIf, hWhile, cs);
   }
@@ -1245,7 +1258,9 @@ void capture_graph(espp_system* s, const IntegrateArgs& ai, bool steps) {
   cudaGraphExec_t ex = nullptr;
   try {
     add_step_loop(s, g, ai, steps);
-    cuda_check(cudaGraphInstantiate(&ex, g, 0), "cudaGraphInstantiate");
+    const cudaError_t e = cudaGraphInstantiate(&ex, g, 0);
+    if (steps) steps_check(e, "cudaGraphInstantiate");
+    cuda_check(e, "cudaGraphInstantiate");
   } catch (...) {
     cudaGraphDestroy(g);
     throw;
@@ -1539,7 +1554,8 @@ void run(espp_system* s, int64_t nsteps) {
   RunSnapshot snap = take_snapshot(s);
   IntegrateArgs ai = run_prologue(s, nsteps, tResort, &snap.ctr);
   IntegrateArgs ag = graph_args(ai);
-  bool steps = steps_wanted(s);
+  const std::string key = graph_key(s, ag);
+  bool steps = steps_wanted(s) && key != s->stepsRefused;
   if (steps) {
     if (!s->stepSync) s->stepSync = dalloc<StepSync>(1);
     if (s->posqAltCap < s->cap) {
@@ -1549,20 +1565,15 @@ void run(espp_system* s, int64_t nsteps) {
     }
     cuda_check(cudaMemsetAsync(s->stepSync, 0, sizeof(StepSync), s->st), "memset");
   }
-  std::string key = graph_key(s, ag) + (steps ? "s" : "k");
-  if (!s->graphExec || key != s->graphKey) {
+  if (!s->graphExec || s->graphKey != key + (steps ? "s" : "k")) {
     try {
       capture_graph(s, ag, steps);
-    } catch (const Fail&) {
-      // no cooperative launch here (or not at this size): the loop of separate kernels
-      if (!steps) throw;
-      cudaGetLastError();
-      s->stepsOff = true;
+    } catch (const StepsRefused&) {
+      s->stepsRefused = key;
       steps = false;
-      key = graph_key(s, ag) + "k";
       capture_graph(s, ag, false);
     }
-    s->graphKey = key;
+    s->graphKey = key + (steps ? "s" : "k");
   }
   cuda_check(cudaGraphLaunch(s->graphExec, s->st), "cudaGraphLaunch");
   cuda_check(cudaEventRecord(s->runEnd, s->st), "event");

@@ -157,6 +157,21 @@ def _chain_bonds(n, beads):
     return np.stack([k, k + 1], 1)
 
 
+def _one_launch(n, prec):
+    """Whether the default lanes of n particles fit the step kernel's one block an SM."""
+    import torch
+
+    lanes = (torch.cuda.get_device_properties(0).multi_processor_count
+             * (1024 if prec == _abi.PREC_MIXED else 640))
+    return n <= 65536 and n * (4 if 4 * n <= lanes else 2) <= lanes
+
+
+def _force_launches(s):
+    k = (ctypes.c_int64 * 8)()
+    call(s.lib, "espp_profile", s.h, None, k)
+    return k[0]
+
+
 # sizes around the edges of the one-launch loop's rules: one block, partial blocks, 4 and 2
 # lanes a particle (23,680 in FP64 and 37,888 in mixed precision on 148 SMs), the last size it
 # takes and the first it does not
@@ -184,7 +199,11 @@ def test_step_loop_matches_host_loop(prec, shape, types, fene, monkeypatch):
             s.fene(30.0, 0.0, 1.5)
         s.langevin(1.0, 1.2)
         for steps in (1, 23, 6):
+            call(s.lib, "espp_set_profiling", s.h, 0)  # zeroes the launch counters
             s.run(steps)
+            # the start-of-run force, then one launch from a re-sort to the next, or one a step
+            one = graph == "1" and _one_launch(n, prec)
+            assert _force_launches(s) == 1 + (s.num_resorts() + 1 if one else steps)
         sims.append(s)
     a, b = (s.particles(np.arange(n)) for s in sims)
     for x, y in zip(a, b):
