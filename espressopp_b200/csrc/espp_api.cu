@@ -68,10 +68,20 @@ void dfree(T*& p) {
   p = nullptr;
 }
 
-// pinned host mirror of what a run reads back
+// pinned host side of the counters, and of what a run reads back
 struct HostState {
+  DevCounters io;
   DevCounters ctr;
   unsigned err;
+  ParticleArrays pa[2];
+};
+
+// small device state of a system, one allocation
+struct DevState {
+  DevCounters ctr;
+  StepSync sync;
+  unsigned err;
+  unsigned ticket;
   ParticleArrays pa[2];
 };
 
@@ -139,11 +149,12 @@ struct espp_system {
   bool idDirty = true;
 
   // device scalars
-  unsigned* err = nullptr;
-  DevCounters* ctr = nullptr;     // device
-  DevCounters* hctr = nullptr;    // pinned host mirror
-  HostState* hstate = nullptr;    // pinned
-  ParticleArrays* d_pa = nullptr; // device: [0] current, [1] re-sort target
+  DevState* dstate = nullptr;
+  unsigned* err = nullptr;        // in dstate, as the next two
+  DevCounters* ctr = nullptr;
+  ParticleArrays* d_pa = nullptr; // [0] current, [1] re-sort target
+  HostState* hstate = nullptr;
+  DevCounters* hctr = nullptr;    // in hstate
   bool paHostValid = true;        // host A/B mirror what d_pa holds
   double* obs = nullptr;
   double* partials = nullptr;
@@ -159,9 +170,6 @@ struct espp_system {
   cudaEvent_t sideBeg = nullptr, sideEnd = nullptr;
   // one-launch step loop of a small system (k_steps)
   std::string stepsRefused;  // graph key for which the GPU refused the cooperative launch
-  StepSync* stepSync = nullptr;
-  int4* posqAlt = nullptr;
-  int posqAltCap = 0;
   int nsm = 0;
   // pre-run snapshot to recover from a Verlet-list overflow inside the graph
   ParticleArrays snap{};
@@ -1219,7 +1227,7 @@ void add_step_loop(espp_system* s, cudaGraph_t g, const IntegrateArgs& ai, bool 
     DevView d = s->view();
     if (!s->has_vl || !s->lj_any) d.nn = s->nnZero;  // no LJ term: bonds only
     steps_check(launch_steps(d, s->precision == ESPP_PREC_MIXED, s->fene, ai, skinHalf,
-                             s->stepSync, s->posqAlt, hIf, hWhile, force_tpp(s), s->nsm, cs),
+                             &s->dstate->sync, hIf, hWhile, force_tpp(s), s->nsm, cs),
                 "step kernel");
   } else {
     launch_decide_graph(s->view(), skinHalf, hIf, hWhile, cs);
@@ -1556,15 +1564,7 @@ void run(espp_system* s, int64_t nsteps) {
   IntegrateArgs ag = graph_args(ai);
   const std::string key = graph_key(s, ag);
   bool steps = steps_wanted(s) && key != s->stepsRefused;
-  if (steps) {
-    if (!s->stepSync) s->stepSync = dalloc<StepSync>(1);
-    if (s->posqAltCap < s->cap) {
-      dfree(s->posqAlt);
-      s->posqAlt = dalloc<int4>(s->cap);
-      s->posqAltCap = s->cap;
-    }
-    cuda_check(cudaMemsetAsync(s->stepSync, 0, sizeof(StepSync), s->st), "memset");
-  }
+  if (steps) cuda_check(cudaMemsetAsync(&s->dstate->sync, 0, sizeof(StepSync), s->st), "memset");
   if (!s->graphExec || s->graphKey != key + (steps ? "s" : "k")) {
     try {
       capture_graph(s, ag, steps);
@@ -1770,7 +1770,6 @@ void destroy(espp_system* s) {
   dfree(s->cellStart);
   dfree(s->scr.cellCount);
   dfree(s->scr.tileSum);
-  dfree(s->scr.ticket);
   dfree(s->id2idx);
   dfree(s->bondStart);
   dfree(s->bondPartner);
@@ -1778,13 +1777,9 @@ void destroy(espp_system* s) {
   dfree(s->halo);
   dfree(s->exclStart);
   dfree(s->exclIds);
-  dfree(s->err);
   destroy_graph(s);
   free_particles(s->snap);
-  dfree(s->stepSync);
-  dfree(s->posqAlt);
-  dfree(s->ctr);
-  dfree(s->d_pa);
+  dfree(s->dstate);
   dfree(s->obs);
   dfree(s->partials);
   dfree(s->d_lj);
@@ -1814,7 +1809,6 @@ void destroy(espp_system* s) {
   if (s->runBeg) cudaEventDestroy(s->runBeg);
   if (s->runLoop) cudaEventDestroy(s->runLoop);
   if (s->runEnd) cudaEventDestroy(s->runEnd);
-  if (s->hctr) cudaFreeHost(s->hctr);
   if (s->hstate) cudaFreeHost(s->hstate);
   if (s->sideBeg) cudaEventDestroy(s->sideBeg);
   if (s->sideEnd) cudaEventDestroy(s->sideEnd);
@@ -1939,19 +1933,17 @@ int espp_system_create(const double box[3], double skin, const int32_t cell_grid
     s->cellStart = dalloc<int32_t>(ncells + 1);
     s->scr.cellCount = dalloc<int32_t>(ncells);
     s->scr.tileSum = dalloc<int32_t>(scan_tiles((int)ncells) + 1);
-    s->scr.ticket = dalloc<unsigned>(1);
+    s->dstate = dalloc<DevState>(1);
+    s->err = &s->dstate->err;
+    s->ctr = &s->dstate->ctr;
+    s->d_pa = s->dstate->pa;
+    s->scr.ticket = &s->dstate->ticket;
+    cuda_check(cudaMemsetAsync(s->dstate, 0, sizeof(DevState), s->st), "memset");
     cuda_check(cudaMemsetAsync(s->scr.cellCount, 0, sizeof(int32_t) * ncells, s->st), "memset");
-    cuda_check(cudaMemsetAsync(s->scr.ticket, 0, sizeof(unsigned), s->st), "memset");
     cuda_check(cudaMemsetAsync(s->cellStart, 0, sizeof(int32_t) * (ncells + 1), s->st), "memset");
-    s->err = dalloc<unsigned>(1);
-    s->ctr = dalloc<DevCounters>(1);
-    s->d_pa = dalloc<ParticleArrays>(2);
     s->obs = dalloc<double>(8);
-    cuda_check(cudaMemsetAsync(s->err, 0, sizeof(unsigned), s->st), "memset");
-    cuda_check(cudaMemsetAsync(s->ctr, 0, sizeof(DevCounters), s->st), "memset");
-    cuda_check(cudaMemsetAsync(s->d_pa, 0, 2 * sizeof(ParticleArrays), s->st), "memset");
-    cuda_check(cudaMallocHost(&s->hctr, sizeof(DevCounters)), "pinned counters");
     cuda_check(cudaMallocHost(&s->hstate, sizeof(HostState)), "pinned state");
+    s->hctr = &s->hstate->io;
     if (const char* g = std::getenv("ESPP_B200_GRAPH")) s->useGraph = std::atoi(g) != 0;
     if (const char* b = std::getenv("ESPP_B200_BRICK")) s->brickAllowed = std::atoi(b) != 0;
     if (const char* b = std::getenv("ESPP_B200_BRICK_BUILD")) s->brickBuild = std::atoi(b) != 0;

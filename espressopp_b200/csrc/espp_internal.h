@@ -239,10 +239,9 @@ void launch_wait_selftest(unsigned* err, long long spins, unsigned long long* ou
 void launch_integrate(const DevView& d, const IntegrateArgs& a, cudaStream_t st);
 // maxDist += sqrt(max |dx|^2); flag = maxDist > skinHalf
 // Every step up to the next re-sort or the end of the run as one cooperative launch; sets the
-// conditionals of the captured loop.  sync: zeroed before the run; posqAlt: second buffer of
-// packed coordinates.
+// conditionals of the captured loop.  sync: zeroed before the run.
 cudaError_t launch_steps(const DevView& d, bool mixed, const FENEParams& fene,
-                         const IntegrateArgs& a, double skinHalf, StepSync* sync, int4* posqAlt,
+                         const IntegrateArgs& a, double skinHalf, StepSync* sync,
                          cudaGraphConditionalHandle hIf, cudaGraphConditionalHandle hWhile,
                          int tpp, int nsm, cudaStream_t st);
 constexpr int kStepParticles = 65536;  // 16-bit list entries in shared memory

@@ -1604,9 +1604,11 @@ struct StepShare {
 template <bool MIXED, int T, bool SINGLE, bool CAPPED, bool FENE>
 __global__ void __launch_bounds__(kStepThreads<MIXED>, 1)
     k_steps(DevView d, FENEParams fp, IntegrateArgs a, double skinHalf, StepSync* sync,
-            int4* posqAlt, cudaGraphConditionalHandle hIf, cudaGraphConditionalHandle hWhile) {
+            cudaGraphConditionalHandle hIf, cudaGraphConditionalHandle hWhile) {
   const ParticleArrays P = d.pa[0];
-  double* const xAlt = d.pa[1].x;  // the re-sort's target is free between re-sorts
+  // the second buffers of the positions: the re-sort's target is free between re-sorts
+  double* const xAlt = d.pa[1].x;
+  int4* const posqAlt = reinterpret_cast<int4*>(d.pa[1].v);
   __shared__ LJPairF sP[kMaxTypes * kMaxTypes];
   __shared__ double smax[kStepThreads<MIXED> / 32];
   if (MIXED && !SINGLE)
@@ -2782,10 +2784,10 @@ void launch_decide_graph(const DevView& d, double skinHalf, cudaGraphConditional
 namespace {
 template <bool MIXED, int T>
 cudaError_t steps_dispatch(const DevView& d, const FENEParams& fp, const IntegrateArgs& a,
-                           double skinHalf, StepSync* sync, int4* posqAlt,
+                           double skinHalf, StepSync* sync,
                            cudaGraphConditionalHandle hIf, cudaGraphConditionalHandle hWhile,
                            int nsm, cudaStream_t st) {
-  using Kernel = void (*)(DevView, FENEParams, IntegrateArgs, double, StepSync*, int4*,
+  using Kernel = void (*)(DevView, FENEParams, IntegrateArgs, double, StepSync*,
                           cudaGraphConditionalHandle, cudaGraphConditionalHandle);
   const bool single = d.ljSingle != 0, capped = d.ljCapped != 0, fene = fp.on != 0;
   Kernel f = nullptr;
@@ -2816,7 +2818,7 @@ cudaError_t steps_dispatch(const DevView& d, const FENEParams& fp, const Integra
   DevView dv = d;
   FENEParams fv = fp;
   IntegrateArgs av = a;
-  void* args[] = {&dv, &fv, &av, &skinHalf, &sync, &posqAlt, &hIf, &hWhile};
+  void* args[] = {&dv, &fv, &av, &skinHalf, &sync, &hIf, &hWhile};
   return cudaLaunchCooperativeKernel((const void*)f, dim3(grid), dim3(block), args, smem, st);
 }
 }  // namespace
@@ -2824,12 +2826,12 @@ cudaError_t steps_dispatch(const DevView& d, const FENEParams& fp, const Integra
 int step_threads(bool mixed) { return mixed ? kStepThreads<true> : kStepThreads<false>; }
 
 cudaError_t launch_steps(const DevView& d, bool mixed, const FENEParams& fp,
-                         const IntegrateArgs& a, double skinHalf, StepSync* sync, int4* posqAlt,
+                         const IntegrateArgs& a, double skinHalf, StepSync* sync,
                          cudaGraphConditionalHandle hIf, cudaGraphConditionalHandle hWhile,
                          int tpp, int nsm, cudaStream_t st) {
 #define ESPP_STEPS(T)                                                                        \
-  return mixed ? steps_dispatch<true, T>(d, fp, a, skinHalf, sync, posqAlt, hIf, hWhile, nsm, st) \
-               : steps_dispatch<false, T>(d, fp, a, skinHalf, sync, posqAlt, hIf, hWhile, nsm, st)
+  return mixed ? steps_dispatch<true, T>(d, fp, a, skinHalf, sync, hIf, hWhile, nsm, st)     \
+               : steps_dispatch<false, T>(d, fp, a, skinHalf, sync, hIf, hWhile, nsm, st)
   switch (tpp) {
     case 1: ESPP_STEPS(1);
     case 2: ESPP_STEPS(2);
