@@ -212,6 +212,85 @@ def test_step_loop_matches_host_loop(prec, shape, types, fene, monkeypatch):
     assert sims[0].builds() == sims[1].builds()
 
 
+# lanes a particle other than the default, lists beyond the step kernel's stage of 104 entries
+# (rc 2.9), capped potential, both forms of CapForce, particles without thermostat
+@pytest.mark.parametrize("prec", [_abi.PREC_FP64, _abi.PREC_MIXED])
+@pytest.mark.parametrize("tpp,rc,caprad,capforce,excluded", [
+    (1, RC, 0.0, None, False), (8, RC, 0.0, None, True), (2, 2.9, 0.0, None, False),
+    (4, 2.9, 0.97, None, True), (8, 2.9, 0.0, None, False), (1, 2.9, 0.97, (1, 40.0), False),
+    (0, RC, 0.97, (1, 30.0), True), (0, RC, 0.0, (2, [15.0, 20.0, 25.0]), True)])
+def test_step_loop_options(prec, tpp, rc, caprad, capforce, excluded, monkeypatch):
+    pos, box = _box_lattice(12, 13, 14, jitter=0.15, seed=6)
+    n = len(pos)
+    vel = mb_velocities(n, 1.2, 5)
+    sims = []
+    for graph in ("0", "1"):
+        monkeypatch.setenv("ESPP_B200_GRAPH", graph)
+        s = _fluid(cuda_lib(), prec, pos, box, vel=vel, rc=rc)
+        if caprad:
+            q = rc ** -6
+            s.lj(0, 0, 1.0, 1.0, rc, 4.0 * (q * q - q), caprad)
+        s.langevin(1.0, 1.2, excl=np.arange(0, n, 5) if excluded else None)
+        if capforce:
+            s.capforce(*capforce)
+        s.integrator(0.002)
+        if tpp:
+            call(s.lib, "espp_set_tpp", s.h, tpp)
+        for steps in (1, 40):
+            call(s.lib, "espp_set_profiling", s.h, 0)
+            s.run(steps)
+            assert _force_launches(s) == 1 + (s.num_resorts() + 1 if graph == "1" else steps)
+        sims.append(s)
+    assert sims[0].num_resorts() == sims[1].num_resorts() >= 1
+    for x, y in zip(*(s.particles(np.arange(n)) for s in sims)):
+        assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("shape", [(20, 20, 20), (33, 33, 33)])
+def test_step_loops_of_two_threads(shape):
+    """Two systems stepped from two threads at once, each in one-launch loops of its own: as one
+    after the other.  The smaller ones are resident together, of the larger ones each fills
+    the GPU."""
+    import threading
+
+    pos, box = _box_lattice(*shape, seed=8)
+    n = len(pos)
+
+    def fresh():
+        out = []
+        for k in range(2):
+            s = _fluid(cuda_lib(), _abi.PREC_MIXED, pos, box, vel=mb_velocities(n, 1.2, k))
+            s.langevin(1.0, 1.2)
+            out.append(s)
+        return out
+
+    def steps(s):
+        for _ in range(12):
+            s.run(15)
+
+    one = fresh()
+    for s in one:
+        steps(s)
+    two = fresh()
+    failed = []
+
+    def job(s):
+        try:
+            steps(s)
+        except RuntimeError as e:
+            failed.append(str(e))
+
+    jobs = [threading.Thread(target=job, args=(s,)) for s in two]
+    for t in jobs:
+        t.start()
+    for t in jobs:
+        t.join()
+    assert not failed
+    for a, b in zip(one, two):
+        for x, y in zip(a.particles(np.arange(n)), b.particles(np.arange(n))):
+            assert np.array_equal(x, y)
+
+
 @pytest.mark.parametrize("tpp", [1, 2, 4, 8])
 def test_mixed_sums_are_fixed_point(tpp):
     """FP32 partial sums are combined in 2^-32 fixed point, nothing is added in FP32 across

@@ -230,3 +230,31 @@ def test_force_of_dimers(itype):
             s.run(0)
             f.append(s.particles(np.arange(2))[2])
         assert np.array_equal(*f), d
+
+
+@pytest.mark.parametrize("prec,tol", [(_abi.PREC_FP64, 1e-12), (_abi.PREC_MIXED, 1e-8)])
+def test_tabulated_bonds_alone(prec, tol):
+    """Bonds with a table and no pair potential: the tabulated pass writes every force itself,
+    over whatever a pass before it left.  Mixed: a force rounds once to 2^-32."""
+    pos, box = lattice(11, 0.8442, 0.1, 9)
+    n = len(pos)
+    k = np.arange(0, n - 1)
+    bonds = np.stack([k, k + 1], 1)[(k + 1) % 11 != 0][::2]  # half of the particles have none
+    r = np.linspace(0.01, 6.0, 500)
+    out = []
+    for lib, p in ((oracle_lib(), _abi.PREC_FP64), (cuda_lib(), prec)):
+        s = Sim(lib, box, 0.3, cell_grid(box, 1.5, 0.3), precision=p, seed=5)
+        s.add(np.arange(n), pos)
+        s.decompose()
+        s.vl(1.5)
+        s.bonds(bonds)
+        s.integrator(0.002)
+        for strength in (300.0, 5.0):
+            _tab_bond(s, _abi.TAB_LINEAR, (r, strength * (r - 1.0) ** 2, -2 * strength * (r - 1.0)))
+            s.run(0)
+        s.run(20)
+        out.append(s.particles(np.arange(n)))
+    (xo, vo, fo, _), (xg, vg, fg, _) = out
+    assert _rel_rms(fg, fo) < 100 * tol and np.max(np.abs(xg - xo)) < 100 * tol
+    free = np.setdiff1d(np.arange(n), bonds)
+    assert len(free) and np.all(fg[free] == 0.0)
