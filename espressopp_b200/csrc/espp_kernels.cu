@@ -697,8 +697,11 @@ constexpr int kBlockW = 4;          // warps a run
 // 33; at 241,133 137 and 142, at 4,096,000 1.97 and 2.17 ms).
 constexpr int kBuildSplit = 100000;
 // List capacity up to which the block form is used.  The capacity is 1.6 times the length
-// expected from the density, and 32 more: lists of 100 entries on average.
-constexpr int kBlockListMax = 192;
+// expected from the density, and 32 more.  Run form / block form in a liquid: 81 / 36 us
+// at 32,768 particles and 191 / 145 at 238,328 with lists of 100 entries (capacity 200), 90 /
+// 90 and 201 / 171 with 114 (216), 110 / 110 and 242 / 243 with 150 (272; the system has
+// changed to the run form).
+constexpr int kBlockListMax = 224;
 
 // Warp that takes row rr of the (2h+1)^2 rows, and its stage in entries.  One cell layer: the
 // centre row, with 29 of an LJ particle's 78 partners on average and 46 at most (counted on

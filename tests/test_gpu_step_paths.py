@@ -61,9 +61,9 @@ def test_build_pair_set(shape, excluded):
     assert g.digest() == o.digest()
 
 
-@pytest.mark.parametrize("rc", [3.2, 3.6, 5.0])
+@pytest.mark.parametrize("rc", [2.6, 2.75, 2.9, 3.2, 3.6, 5.0])
 def test_long_lists(rc):
-    """Lists of a capacity above 192 entries take the run form."""
+    """Lists up to the block form's last capacity (224) and beyond it."""
     pos, box = _box_lattice(17, 17, 18, jitter=0.2, seed=4)
     g = _fluid(cuda_lib(), _abi.PREC_MIXED, pos, box, rc=rc)
     o = _fluid(oracle_lib(), _abi.PREC_FP64, pos, box, rc=rc)
