@@ -63,9 +63,8 @@ STEP_FLOPS = 24.0 * N_HALF
 # force kernel: packed coordinates read 12 + 4 B per half-list pair + int64 F write 24
 FORCE_BYTES = 12.0 + 4.0 * N_HALF + 24.0
 # DRAM bytes (read + write) per particle of one force-kernel launch, measured by ncu on
-# the 1,000,000-particle case (profiles/force_mixed_lj_1M_ncu.txt: 345.0 MB + 6.7 MB for
-# the global-list kernel); traffic grows in proportion to the particle count at fixed
-# density
+# the 1,000,000-particle case (profiles/force_mixed_lj_1M_ncu.txt: 340 MB + 6 to 9 MB for the
+# global-list kernel); traffic grows in proportion to the particle count at fixed density
 FORCE_TRAFFIC_PER_PARTICLE = {"k_force_mixed": 347.4}
 
 
@@ -1199,7 +1198,7 @@ def main():
                     help="threads per particle of the global-list force kernel")
     ap.add_argument("--layout", default="auto",
                     choices=["auto", "global", "brick", "global-brick-build"],
-                    help="list layout: autotuned, global per-particle lists (per-cell build), "
+                    help="list layout: autotuned, global per-particle lists, "
                          "brick windows, global lists built by brick windows")
     args = ap.parse_args()
     if args.warmup < 3:

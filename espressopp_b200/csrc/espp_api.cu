@@ -976,10 +976,10 @@ constexpr double kApartMs = 0.006;
 
 // Main pair + FENE kernel (list counts zeroed when no LJ pair is set), then the
 // tabulated pair and bond forces added to its output.  The descriptor and the site network of a
-// learned potential and the terms of the angles read positions only, and none of these kernels
-// fills the GPU at 50,000 particles: they run beside the others on a second stream (branches of
-// a captured graph).  Sums are added in the same order as on one stream.  A step of
-// 50,000 sites takes 115 us this way, 124 on one stream.
+// learned potential read positions only, and none of these kernels fills the GPU at 50,000
+// particles: the two run on a second stream (a branch of a captured graph) beside the main, the
+// tabulated and the angle kernels.  Sums are added in the same order as on one stream.  A step
+// of 50,000 sites takes 115 us this way, 124 on one stream.
 void launch_all_forces(espp_system* s, cudaStream_t st) {
   DevView d = s->view();
   const bool mixed = s->precision == ESPP_PREC_MIXED;

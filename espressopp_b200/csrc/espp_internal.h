@@ -218,7 +218,7 @@ void launch_fold_bin(const DevView& d, RebuildScratch& s, bool fold, cudaStream_
 void launch_sort_cells(const DevView& d, RebuildScratch& s, cudaStream_t st);
 int resort_launches(const DevView& d);  // kernels of one re-sort without the list build
 // Verlet list in the global form; fresh: the particles were binned at their current
-// positions (the run form may then be used).
+// positions (no candidate's cell need be checked then).
 void launch_build_nl(const DevView& d, double cutsq, bool fresh, cudaStream_t st);
 void launch_posq(const DevView& d, cudaStream_t st);
 void launch_xrel(const DevView& d, cudaStream_t st);

@@ -275,8 +275,8 @@ __device__ __forceinline__ void swap_when_last(const DevView& d, const RebuildSc
 // costs (7.5 us for 32,768 particles, 18 as four kernels).  Its registers and the sort's
 // barrier leave a third of the threads in flight that a plain gather has, so large systems
 // (kMoveApart) write the order and move in a kernel of its own (100 us fused, 82 apart at a
-// million particles).  A cell's serial insertion sort by one lane took 115 us at 2,028
-// particles in 16 large cells, the ranking 8.
+// million particles).  The ranking takes 8 us at 2,028 particles in 16 large cells, a serial
+// insertion sort by one lane a cell 115.
 constexpr int kSortThreads = 256;
 constexpr int kSortKeys = 1024;  // particles of a block ranked in shared memory
 constexpr int kMoveApart = 150000;
@@ -688,13 +688,13 @@ __global__ void __launch_bounds__(kRunWarps * 32) k_build_nl_run(DevView d, doub
 // scans them, keeps its partners in its own stage (transposed: entry-major, no bank conflicts)
 // and the block writes the lists once, in whole blocks of 8.
 // A warp alone spends about 7 cycles an instruction on this work, so a run handled by one
-// warp lasts 60 us however few particles there are.  Measured, run form against this one:
-// 62 / 20 us at 2,028 particles, 64 / 33 at 32,768, 157 / 137 at 241,133, 2.03 / 1.97 ms at
-// 4,096,000 (issue bound in both: about 400 instructions a particle), 49 / 24 at the
+// warp lasts 60 us however few particles there are.  Run form / this one: 71 / 18 us at 2,028
+// particles, 69 / 32 at 32,768, 163 / 129 at 241,133, 540 / 479 at a million, 2.02 / 1.88 ms at
+// 4,096,000 (issue bound in both: about 320 instructions a particle here), 48 / 28 at a
 // 40,000-bead melt.
-constexpr int kBlockW = 4;          // warps a run
-// Particles up to which two blocks share a run (SPLIT; one block a run: 36 us at 32,768, two:
-// 33; at 241,133 137 and 142, at 4,096,000 1.97 and 2.17 ms).
+constexpr int kBlockW = 4;  // warps a run
+// Particles up to which two blocks share a run (SPLIT).  One block a run / two: 22 / 18 us at
+// 2,028, 34 / 32 at 32,768, 129 / 135 at 241,133, 1.88 / 2.07 ms at 4,096,000.
 constexpr int kBuildSplit = 100000;
 // List capacity up to which the block form is used.  The capacity is 1.6 times the length
 // expected from the density, and 32 more.  Run form / block form in a liquid: 81 / 36 us
@@ -1746,10 +1746,10 @@ __global__ void __launch_bounds__(kStepThreads<MIXED>, 1)
 // virial r.F and its tensor (VerletListInteractionTemplate.hpp:274-331) over each listed pair
 // once (j > i).  T lanes a particle (ListShare), a block of 256 threads 256 particles in T
 // rounds; the minimum image is skipped where k_force_fp64 skips it.  Bound by the FP64 pipe and
-// the latency of the gathers: 423 us a pass before, 277 (energy) and 321 (virial tensor) now at
-// a million particles.  Two lanes at every size; a call with four takes 49.0 us (energy) and
-// 62.0 (virial) against 47.4 and 53.5 at 8,000 particles, 96 and 114 against 88 and 111 at
-// 216,000.
+// the latency of the gathers: 277 us (energy) and 321 (virial tensor) at a million particles,
+// 423 with one lane that loads entry by entry.  Two lanes at every size; a call with four takes
+// 49.0 us (energy) and 62.0 (virial) against 47.4 and 53.5 at 8,000 particles, 96 and 114
+// against 88 and 111 at 216,000.
 constexpr int kObsLanes = 2;
 template <bool ENERGY, bool SINGLE>
 __global__ void __launch_bounds__(kBlock, 3) k_lj_obs(DevView d, double* partials) {
@@ -1918,7 +1918,7 @@ __device__ __forceinline__ int rdf_bin(const DevView& d, double ex, double ey, d
 // the minimum image.  17 instructions a pair, all of them FP32 or integer, against 40 in FP64.
 // Counts go to `copies` copies of the histogram in shared memory, a lane's copy by its bank
 // (no bank conflicts with 32), flushed with one global atomic per non-empty bin.
-// Bound by issue: a call at 32,768 particles and 256 bins took 1,617 us in FP64, now 742.
+// Bound by issue: 743 us a call at 32,768 particles and 256 bins, 1,617 with FP64 for every pair.
 template <bool SMEM, bool FAST>
 __global__ void __launch_bounds__(kRdfTile) k_rdf(DevView d, int rdfN, int ntiles, double dr,
                                                   float far, int copies, unsigned long long* hist) {

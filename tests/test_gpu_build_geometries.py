@@ -4,9 +4,10 @@ many x-cells) and its x-cell range with periodic wrap, against the FP64 oracle
 (VerletList.cpp:274-450):
 
 * a dilute gas (0.4 particles per cell): groups span many cells and split by span;
-* the smallest grid the run form takes in x (3 cells) with long y and z;
+* the smallest grid in x (3 cells) with long y and z;
 * a slab: particles only in a third of the box, so most rows are empty;
-* cells just above the cutoff (0.2 %: the run form; 0.05 %: the per-cell form);
+* cells just above the cutoff (0.2 %: the plain form; 0.05 %: each candidate's cell checked);
+* rows of hundreds of cells with few particles, and cells of many cutoffs;
 and a grid of 2 cells in one dimension, which the GPU storage refuses.
 Each compares the sorted id-pair sets, the pair digests and the mixed-precision forces.
 """
@@ -98,7 +99,7 @@ def test_slab_with_empty_rows():
 
 @pytest.mark.parametrize("edge", [2.8 * 1.002, 2.8 * 1.0005])
 def test_cells_just_above_the_cutoff(edge):
-    """Edges 0.2 % above the cutoff take the run form, 0.05 % the per-cell form."""
+    """Edges 0.2 % above the cutoff need no check of a candidate's cell, 0.05 % do."""
     rng = np.random.Generator(np.random.PCG64(24))
     grid = [10, 9, 11]
     box = np.array(grid, float) * edge
